@@ -159,8 +159,6 @@ struct Dev {
   // and whether its full fan of elements closes (360 degrees)
   int *iweg, *iwet, *inod;
   unsigned char *kfull;
-  float4 *cg4[2];                 // device-wide CG: {r, w = A D^-1 r, s, 1/diag} per row, two generations
-  float2 *cg2;                    // device-wide CG: {p, e} per row
   // element system written by the column kernel, 12 floats per element:
   // hia (3x3, row-major, [e*12 + 3i+j]) then hik ([e*12 + 9 + i])
   float *hia;

@@ -258,7 +258,7 @@ struct Arena {
 // ---------------------------------------------------------------------------
 // the model
 // ---------------------------------------------------------------------------
-static const int kMaxZetaClasses = 10;  // zeta launch classes: 2 variants x cluster sizes 1..16
+static const int kMaxZetaClasses = 10;  // zeta launch classes (cluster sizes 1..16)
 static int next_pow2(int n);
 
 struct shygpu_model {
@@ -315,8 +315,7 @@ struct shygpu_model {
   cudaStream_t side[kMaxZetaClasses] = {};
   cudaEvent_t ev_fork = nullptr, ev_join[kMaxZetaClasses] = {};
   std::vector<int> rowptr_h, col_h;  // global CSR pattern (host copy)
-  int *zmap_ptrs[3] = {nullptr, nullptr, nullptr};
-  ZetaMaps zm;
+  std::vector<float> xy_h;           // node coordinates, x and y in turn (the resident solver's shares)
   float inner_rtol = 1e-4f;
   float tol_frac = 0.75f;          // measured: 0.75 saves 6% of the solve against 0.25 with no extra refinement
   // graphs keyed by (cur, sc_cur)
@@ -342,28 +341,29 @@ static void drop_graphs(shygpu_model *m) {
       if (m->graph[a][b]) { cudaGraphExecDestroy(m->graph[a][b]); m->graph[a][b] = nullptr; }
 }
 
-static int check_cluster_shape(int CL, int threads, size_t smem);
+static int check_cluster_shape(int CL, int threads);
 
-// ---------------------------------------------------------------------------
-// Launch plan of the zeta solver.  Basins are grouped into classes with one
-// cluster shape each (at most 1250 rows per CTA, 640 threads); the
-// classes' launches run concurrently.  The shared-memory variant keeps each
-// CTA's rows (row pointers, local columns, FP32 values) and seven FP32
-// vectors plus a halo in shared memory; it serves symmetric systems whose
-// slices fit 227 KB, the global-memory variant the rest.
-// ---------------------------------------------------------------------------
-static const size_t kSmemMax = 227 * 1024;
-
+// Zeta launch plan.  A symmetric model runs in one cooperative launch over
+// the device: the resident solver (k_zeta_team), or the streaming one
+// (k_zeta_grid) when a basin does not fit on chip or its tiles are asked
+// for.  Other systems run k_zeta, a cluster per basin with vectors in global
+// memory, in one launch per cluster size on streams of their own.
 static void free_zeta_plan(shygpu_model *m) {
-  for (int *&p : m->zmap_ptrs) { if (p) cudaFree(p); p = nullptr; }
-  m->zm = ZetaMaps();
   for (ZetaClass &c : m->zcl) {
     if (c.d_blist) cudaFree(c.d_blist);
+    if (c.team) {
+      const TeamPlan &t = c.tp;
+      for (const void *p : {(const void *)t.mem, (const void *)t.cptr, (const void *)t.clist, (const void *)t.rows,
+                            (const void *)t.dpos, (const void *)t.ghost, (const void *)t.lcol, (const void *)t.tcol,
+                            (const void *)t.tptr, (const void *)t.tslot, (const void *)t.tval, (const void *)t.word,
+                            (const void *)t.part, (const void *)t.ctr, (const void *)t.cta_cnt})
+        cudaFree((void *)p);
+    }
     if (c.grid) {
       cudaFree((void *)c.gp.tile); cudaFree((void *)c.gp.btile); cudaFree((void *)c.gp.cslot);
       cudaFree((void *)c.gp.cnslot); cudaFree((void *)c.gp.cowner);
       cudaFree((void *)c.gp.cptr); cudaFree((void *)c.gp.clist);
-      cudaFree(c.gp.partial); cudaFree(c.gp.ctr);
+      cudaFree(c.gp.partial); cudaFree(c.gp.ctr); cudaFree(c.gp.cg4[0]); cudaFree(c.gp.cg4[1]);
       cudaFree((void *)c.gp.ecol16); cudaFree((void *)c.gp.ecol32); cudaFree((void *)c.gp.eslot);
       cudaFree(c.gp.eval); cudaFree((void *)c.gp.xptr); cudaFree((void *)c.gp.xcol);
       cudaFree((void *)c.gp.xslot); cudaFree(c.gp.xval); cudaFree(c.gp.sd); cudaFree(c.gp.ecor);
@@ -522,34 +522,179 @@ static int build_grid_class(shygpu_model *m) {
     CUDA_TRY(cudaMalloc(&c.gp.ecor, sizeof(float) * (NKN + 8)));
     CUDA_TRY(cudaMemset(c.gp.ecor, 0, sizeof(float) * (NKN + 8)));
   }
+  for (float4 *&p : c.gp.cg4) {
+    CUDA_TRY(cudaMalloc(&p, sizeof(float4) * NKN));
+    CUDA_TRY(cudaMemset(p, 0, sizeof(float4) * NKN));
+  }
   CUDA_TRY(cudaMalloc(&c.gp.partial, sizeof(double) * 8 * std::max<size_t>(tile.size(), 1)));
   CUDA_TRY(cudaMalloc(&c.gp.ctr, 8 * sizeof(unsigned)));
   CUDA_TRY(cudaMemset(c.gp.ctr, 0, 8 * sizeof(unsigned)));
   return SHY_OK;
 }
 
-// rows of CTA q of basin bp for cluster size CL
-static inline void cta_rows(const BasinPar &bp, int CL, int q, int &a, int &e) {
-  const int cb = (bp.nk + CL - 1) / CL;
-  a = bp.k0 + std::min(bp.nk, q * cb);
-  e = bp.k0 + std::min(bp.nk, (q + 1) * cb);
-}
-
-// sorted non-local columns of the rows a..e
-static std::vector<int> halo_of(const shygpu_model *m, int a, int e) {
-  std::vector<int> halo;
-  for (int s = m->rowptr_h[a]; s < m->rowptr_h[e]; s++) {
-    const int c = m->col_h[s];
-    if (c < a || c >= e) halo.push_back(c);
+// nodes ord[lo, hi) cut into T compact patches of nearly equal size by
+// recursive bisection of their coordinates, across the longer side; patch r
+// of the T holds ord[cut[r], cut[r+1])
+static void bisect_nodes(std::vector<int> &ord, const float *xy, int lo, int hi, int r, int T, std::vector<int> &cut) {
+  if (T == 1) {
+    cut[r] = lo;
+    std::sort(ord.begin() + lo, ord.begin() + hi);   // rows in order: gathers of neighbours stay local
+    return;
   }
-  std::sort(halo.begin(), halo.end());
-  halo.erase(std::unique(halo.begin(), halo.end()), halo.end());
-  return halo;
+  float a[2] = {INFINITY, INFINITY}, b[2] = {-INFINITY, -INFINITY};
+  for (int i = lo; i < hi; i++)
+    for (int c = 0; c < 2; c++) {
+      a[c] = std::min(a[c], xy[2 * (size_t)ord[i] + c]);
+      b[c] = std::max(b[c], xy[2 * (size_t)ord[i] + c]);
+    }
+  const int c = b[1] - a[1] > b[0] - a[0] ? 1 : 0;
+  const int T1 = T / 2, mid = lo + (int)((long long)(hi - lo) * T1 / T);
+  std::nth_element(ord.begin() + lo, ord.begin() + mid, ord.begin() + hi, [&](int p, int q) {
+    const float u = xy[2 * (size_t)p + c], v = xy[2 * (size_t)q + c];
+    return u != v ? u < v : p < q;
+  });
+  bisect_nodes(ord, xy, lo, mid, r, T1, cut);
+  bisect_nodes(ord, xy, mid, hi, r + T1, T - T1, cut);
 }
 
-static size_t sm_bytes(const ZetaShape &zs) {
-  size_t b = (size_t)4 * (zs.chunk + 1) + (size_t)8 * zs.nnzcap + (size_t)28 * zs.chunk + (size_t)4 * zs.halocap;
-  return (b + 15) & ~(size_t)15;
+// The resident class: every basin in one cooperative launch of k_zeta_team.
+// A basin's team has as many CTAs as its rows need (so its shares and sums
+// depend on it alone); teams are dealt to the CTAs widest first, each to the
+// CTAs that are free soonest, in one order common to all CTAs (so no two
+// CTAs wait for each other's later work).  Returns SHY_EARG when a basin
+// needs more CTAs than are resident or a share has more ghosts than a CTA
+// holds.
+static int build_team_class(shygpu_model *m) {
+  const int cap = zeta_team_capacity(), TR = zeta_team_rows(), NKN = m->NKN;
+  if (cap < 1) return fail(SHY_ECUDA, "zeta resident solver: no resident CTA fits the device");
+  std::vector<TeamMember> mem;
+  std::vector<int> ord(NKN), cut, first(m->nbasin + 1, 0);
+  for (int i = 0; i < NKN; i++) ord[i] = i;
+  long long ctas = 0;
+  for (int b = 0; b < m->nbasin; b++) {
+    const BasinPar &bp = m->par[b];
+    const int rows = zeta_team_share(bp.nk), T = (bp.nk + rows - 1) / rows;
+    if (T > cap) return fail(SHY_EARG, "zeta resident solver: basin %d needs %d CTAs, %d are resident", b, T, cap);
+    cut.assign(T + 1, bp.k0 + bp.nk);
+    bisect_nodes(ord, m->xy_h.data(), bp.k0, bp.k0 + bp.nk, 0, T, cut);
+    const int slot0 = (int)mem.size();
+    for (int r = 0; r < T; r++) mem.push_back(TeamMember{b, T, r, slot0, cut[r], cut[r + 1] - cut[r], 0, 0});
+    first[b + 1] = (int)mem.size();
+    ctas += T;
+  }
+  // shares: ghosts in row order, local columns, tails
+  std::vector<int> dpos(NKN), ghost, local(NKN), own(NKN), seen(NKN, -1), tptr, tslot;
+  std::vector<unsigned short> lcol((size_t)8 * NKN), tcol;
+  std::vector<char> sent(NKN, 0);
+  for (size_t q = 0; q < mem.size(); q++)
+    for (int j = 0; j < mem[q].nrow; j++) { own[ord[mem[q].row0 + j]] = (int)q; local[ord[mem[q].row0 + j]] = j; }
+  bool tail = false;
+  for (int i = 0; i < NKN && !tail; i++) tail = m->rowptr_h[i + 1] - m->rowptr_h[i] > 9;
+  if (tail) tptr.assign(NKN + 1, 0);
+  std::vector<int> gidx(NKN, 0), gl;
+  for (size_t q = 0; q < mem.size(); q++) {
+    TeamMember &M = mem[q];
+    gl.clear();
+    for (int j = 0; j < M.nrow; j++) {
+      const int i = ord[M.row0 + j];
+      for (int s = m->rowptr_h[i]; s < m->rowptr_h[i + 1]; s++) {
+        const int c = m->col_h[s];
+        if (own[c] != (int)q && seen[c] != (int)q) { seen[c] = (int)q; gl.push_back(c); sent[c] = 1; }
+      }
+    }
+    if ((int)gl.size() > zeta_team_ghosts())
+      return fail(SHY_EARG, "zeta resident solver: a share of %d rows has %d ghosts", M.nrow, (int)gl.size());
+    std::sort(gl.begin(), gl.end());
+    M.ghost0 = (int)ghost.size();
+    M.nghost = (int)gl.size();
+    for (size_t g = 0; g < gl.size(); g++) gidx[gl[g]] = TR + (int)g;
+    ghost.insert(ghost.end(), gl.begin(), gl.end());
+    for (int j = 0; j < M.nrow; j++) {
+      const int i = ord[M.row0 + j], s0 = m->rowptr_h[i];
+      unsigned short *lc = &lcol[(size_t)8 * (M.row0 + j)];
+      int n = 0, dp = 0;
+      for (int s = s0; s < m->rowptr_h[i + 1]; s++) {
+        const int c = m->col_h[s];
+        if (c == i) { dp = s - s0; continue; }
+        const int l = own[c] == (int)q ? local[c] : gidx[c];
+        if (n < 8) lc[n] = (unsigned short)(4 * l);
+        else { tcol.push_back((unsigned short)l); tslot.push_back(s); }
+        n++;
+      }
+      for (int k = n; k < 8; k++) lc[k] = (unsigned short)(4 * j);
+      dpos[M.row0 + j] = dp | n << 8;
+      if (tail) tptr[M.row0 + j + 1] = (int)tcol.size();
+    }
+  }
+  for (int &i : ord)
+    if (sent[i]) i |= (int)0x80000000u;
+  // teams to CTAs
+  const int G = (int)std::min<long long>(cap, ctas);
+  std::vector<int> job(m->nbasin);
+  for (int b = 0; b < m->nbasin; b++) job[b] = b;
+  std::stable_sort(job.begin(), job.end(), [&](int x, int y) { return first[x + 1] - first[x] > first[y + 1] - first[y]; });
+  typedef std::pair<int, int> Load;                  // teams worked so far, CTA
+  std::priority_queue<Load, std::vector<Load>, std::greater<Load>> heap;
+  for (int c = 0; c < G; c++) heap.push(Load(0, c));
+  std::vector<std::vector<int>> ctl(G);
+  std::vector<int> who;
+  for (int b : job) {
+    int done = 0;
+    who.clear();
+    for (int q = first[b]; q < first[b + 1]; q++) {
+      done = std::max(done, heap.top().first);
+      who.push_back(heap.top().second);
+      heap.pop();
+    }
+    for (size_t r = 0; r < who.size(); r++) {
+      ctl[who[r]].push_back(first[b] + (int)r);
+      heap.push(Load(done + 1, who[r]));
+    }
+  }
+  std::vector<int> cptr(G + 1, 0), clist;
+  for (int c = 0; c < G; c++) {
+    clist.insert(clist.end(), ctl[c].begin(), ctl[c].end());
+    cptr[c + 1] = (int)clist.size();
+  }
+  m->zcl.emplace_back();
+  ZetaClass &c = m->zcl.back();
+  c.team = true;
+  c.G = G;
+  c.CL = c.threads = 0;
+  for (int i = 0; i < m->nbasin; i++) c.basins.push_back(i);
+  TeamPlan &t = c.tp;
+  t.nslot = (int)mem.size() + 1;                     // the last: the phantom of the timeout test
+  t.phantom = m->zbar_test ? 1 : 0;
+  t.spin_limit = m->zbar_test ? (1LL << 12) : zeta_team_spin_limit();
+  auto up = [&](auto &dst, auto &h) {
+    typename std::decay<decltype(h[0])>::type *p = nullptr;
+    const int st = upload_plan(&p, h);
+    dst = p;
+    return st;
+  };
+  ST_TRY(up(t.mem, mem));
+  ST_TRY(up(t.cptr, cptr));
+  ST_TRY(up(t.clist, clist));
+  ST_TRY(up(t.rows, ord));
+  ST_TRY(up(t.dpos, dpos));
+  ST_TRY(up(t.ghost, ghost));
+  ST_TRY(up(t.lcol, lcol));
+  if (tail) {
+    ST_TRY(up(t.tptr, tptr));
+    ST_TRY(up(t.tcol, tcol));
+    ST_TRY(up(t.tslot, tslot));
+    CUDA_TRY(cudaMalloc(&t.tval, sizeof(float) * tcol.size()));
+  }
+  const size_t nw = (size_t)4 * NKN, np = (size_t)4 * kTeamSlotWords * t.nslot;
+  CUDA_TRY(cudaMalloc(&t.word, sizeof(unsigned long long) * nw));
+  CUDA_TRY(cudaMemset(t.word, 0, sizeof(unsigned long long) * nw));
+  CUDA_TRY(cudaMalloc(&t.part, sizeof(unsigned long long) * np));
+  CUDA_TRY(cudaMemset(t.part, 0, sizeof(unsigned long long) * np));
+  CUDA_TRY(cudaMalloc(&t.ctr, sizeof(unsigned)));
+  CUDA_TRY(cudaMemset(t.ctr, 0, sizeof(unsigned)));
+  CUDA_TRY(cudaMalloc(&t.cta_cnt, sizeof(unsigned) * G));
+  CUDA_TRY(cudaMemset(t.cta_cnt, 0, sizeof(unsigned) * G));
+  return SHY_OK;
 }
 
 static int build_zeta_plan_impl(shygpu_model *m, int forceCL, int forceThreads);
@@ -565,25 +710,16 @@ static int build_zeta_plan(shygpu_model *m, int forceCL, int forceThreads) {
 static int build_zeta_plan_impl(shygpu_model *m, int forceCL, int forceThreads) {
   free_zeta_plan(m);
   const int NKN = m->NKN;
-  // the device-wide solver when asked for, or when a basin of a symmetric
-  // system is too large for the shared-memory cluster solver
-  bool grid = m->sym && m->zvariant == 2 && forceCL <= 0;
-  if (m->sym && m->zvariant == 1 && forceCL <= 0)
-    for (int b = 0; b < m->nbasin && !grid; b++) {
-      const BasinPar &bp = m->par[b];
-      const int CL = std::min(16, next_pow2((bp.nk + 1249) / 1250));
-      ZetaShape zs;
-      for (int q = 0; q < CL; q++) {
-        int a, e;
-        cta_rows(bp, CL, q, a, e);
-        zs.chunk = std::max(zs.chunk, e - a);
-        zs.nnzcap = std::max(zs.nnzcap, m->rowptr_h[e] - m->rowptr_h[a]);
-        zs.halocap = std::max(zs.halocap, (int)halo_of(m, a, e).size());
-      }
-      if (sm_bytes(zs) > kSmemMax) grid = true;
+  // symmetric systems (zeta_variant 1 and 2): the resident solver where every
+  // basin fits it, else, or when its tiles are asked for, the streaming
+  // device-wide solver
+  if (m->sym && m->zvariant && forceCL <= 0) {
+    int st = SHY_EARG;
+    if (!m->zstage && (m->ztile_rows == 0 || m->ztile_rows == zeta_grid_tile_rows())) st = build_team_class(m);
+    if (st == SHY_EARG) {
+      free_zeta_plan(m);
+      st = build_grid_class(m);
     }
-  if (grid) {
-    const int st = build_grid_class(m);
     if (st == SHY_OK) {
       m->zforce_CL = forceCL;
       m->zforce_threads = forceThreads;
@@ -592,96 +728,30 @@ static int build_zeta_plan_impl(shygpu_model *m, int forceCL, int forceThreads) 
     if (st != SHY_EARG) return st;
     free_zeta_plan(m);   // too many basins per CTA: fall back to cluster classes
   }
-  std::vector<int> loc(m->rowptr_h[NKN], 0);
-  std::vector<std::vector<int>> pushl(NKN);
+  // one cluster per basin, classes by cluster size; the thread count is one
+  // for all, so that the reduction order of a basin is the same alone and in
+  // any batch
+  int maxCL = 1;
   for (int b = 0; b < m->nbasin; b++) {
-    const BasinPar &bp = m->par[b];
-    int CL, th;
-    if (forceCL > 0) { CL = forceCL; th = forceThreads; }
-    else {
-      // the thread count depends on nothing but the variant, so that the
-      // reduction order of a basin is the same alone and in any batch
-      CL = std::min(16, next_pow2((bp.nk + 1249) / 1250));
-      th = 640;
-    }
-    bool sm = m->sym && m->zvariant;
-    ZetaShape zs;
-    zs.CL = CL; zs.threads = th;
-    std::vector<std::vector<int>> halos(CL);
-    if (sm) {
-      for (int q = 0; q < CL; q++) {
-        int a, e;
-        cta_rows(bp, CL, q, a, e);
-        zs.chunk = std::max(zs.chunk, e - a);
-        zs.nnzcap = std::max(zs.nnzcap, m->rowptr_h[e] - m->rowptr_h[a]);
-        halos[q] = halo_of(m, a, e);
-        zs.halocap = std::max(zs.halocap, (int)halos[q].size());
-      }
-      sm = sm_bytes(zs) <= kSmemMax;
-    }
-    if (!sm && forceCL <= 0) { CL = std::min(16, next_pow2((bp.nk + 4095) / 4096)); th = 1024; }
-    // the class of this variant and cluster size (its CTAs take the largest
-    // thread count any of its basins wants)
+    const int CL = forceCL > 0 ? forceCL : std::min(16, next_pow2((m->par[b].nk + 4095) / 4096));
+    const int th = forceCL > 0 ? forceThreads : 1024;
     ZetaClass *cls = nullptr;
     for (ZetaClass &c : m->zcl)
-      if (c.sm == sm && c.CL == CL) cls = &c;
+      if (c.CL == CL) cls = &c;
     if (!cls) {
       m->zcl.emplace_back();
       cls = &m->zcl.back();
-      cls->sm = sm; cls->CL = CL; cls->threads = th;
-      cls->zs.CL = CL;
+      cls->CL = CL;
+      cls->threads = th;
     }
-    cls->threads = std::max(cls->threads, th);
-    cls->zs.threads = cls->threads;
     cls->basins.push_back(b);
-    if (sm) {
-      cls->zs.chunk = std::max(cls->zs.chunk, zs.chunk);
-      cls->zs.nnzcap = std::max(cls->zs.nnzcap, zs.nnzcap);
-      cls->zs.halocap = std::max(cls->zs.halocap, zs.halocap);
-      for (int q = 0; q < CL; q++) {
-        int a, e;
-        cta_rows(bp, CL, q, a, e);
-        const int nloc = e - a;
-        const std::vector<int> &halo = halos[q];
-        for (int s = m->rowptr_h[a]; s < m->rowptr_h[e]; s++) {
-          const int c = m->col_h[s];
-          if (c >= a && c < e) loc[s] = c - a;
-          else loc[s] = nloc + (int)(std::lower_bound(halo.begin(), halo.end(), c) - halo.begin());
-        }
-        for (size_t h = 0; h < halo.size(); h++)   // the owner of halo[h] pushes into slot nloc+h of q
-          pushl[halo[h]].push_back((q << 24) | (nloc + (int)h));
-      }
-    }
+    maxCL = std::max(maxCL, CL);
   }
-  // validate every class shape (occupancy with its shared memory)
-  size_t maxsm = 0;
-  int maxCL = 1;
-  for (ZetaClass &c : m->zcl) {
-    if (c.sm) { c.zs.smem = sm_bytes(c.zs); maxsm = std::max(maxsm, c.zs.smem); }
-    maxCL = std::max(maxCL, c.CL);
-  }
-  for (ZetaClass &c : m->zcl) ST_TRY(check_cluster_shape(c.CL, c.threads, c.sm ? c.zs.smem : 0));
-  if (maxsm > 0 || maxCL > 8) {
-    cudaError_t e = zeta_kernel_setup(maxCL, maxsm);
+  for (ZetaClass &c : m->zcl) ST_TRY(check_cluster_shape(c.CL, c.threads));
+  if (maxCL > 8) {
+    cudaError_t e = zeta_kernel_setup(maxCL);
     if (e != cudaSuccess) return fail(SHY_ECUDA, "zeta kernel setup: %s", cudaGetErrorString(e));
   }
-  // maps and basin lists on the device
-  std::vector<int> pptr(NKN + 1, 0), push;
-  for (int i = 0; i < NKN; i++) {
-    pptr[i + 1] = pptr[i] + (int)pushl[i].size();
-    push.insert(push.end(), pushl[i].begin(), pushl[i].end());
-  }
-  int *dl = nullptr, *dp = nullptr, *dq = nullptr;
-  CUDA_TRY(cudaMalloc(&dl, sizeof(int) * std::max<size_t>(loc.size(), 1)));
-  m->zmap_ptrs[0] = dl;
-  CUDA_TRY(cudaMalloc(&dp, sizeof(int) * pptr.size()));
-  m->zmap_ptrs[1] = dp;
-  CUDA_TRY(cudaMalloc(&dq, sizeof(int) * std::max<size_t>(push.size(), 1)));
-  m->zmap_ptrs[2] = dq;
-  CUDA_TRY(cudaMemcpy(dl, loc.data(), sizeof(int) * loc.size(), cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemcpy(dp, pptr.data(), sizeof(int) * pptr.size(), cudaMemcpyHostToDevice));
-  if (!push.empty()) CUDA_TRY(cudaMemcpy(dq, push.data(), sizeof(int) * push.size(), cudaMemcpyHostToDevice));
-  m->zm.loc = dl; m->zm.push_ptr = dp; m->zm.push = dq;
   for (ZetaClass &c : m->zcl) {
     CUDA_TRY(cudaMalloc(&c.d_blist, sizeof(int) * c.basins.size()));
     CUDA_TRY(cudaMemcpy(c.d_blist, c.basins.data(), sizeof(int) * c.basins.size(), cudaMemcpyHostToDevice));
@@ -703,8 +773,8 @@ static int launch_zeta_plan(shygpu_model *m, const Dev &d, ZetaArgs za) {
     cudaStream_t st = nc > 1 ? m->side[i] : m->stream;
     if (nc > 1) CUDA_TRY(cudaStreamWaitEvent(st, m->ev_fork, 0));
     za.blist = c.d_blist;
-    cudaError_t e = c.grid ? launch_zeta_grid(d, za, c.gp, c.G, c.staged, c.gsmem, st)
-                  : c.sm   ? launch_zeta_sm(d, za, c.zs, m->zm, (int)c.basins.size(), st)
+    cudaError_t e = c.team ? launch_zeta_team(d, za, c.tp, c.G, st)
+                  : c.grid ? launch_zeta_grid(d, za, c.gp, c.G, c.staged, c.gsmem, st)
                            : launch_zeta(d, za, c.CL, c.threads, (int)c.basins.size(), st);
     if (e != cudaSuccess) return fail(SHY_ECUDA, "zeta solve launch: %s", cudaGetErrorString(e));
     if (nc > 1) {
@@ -829,11 +899,11 @@ extern "C" int shygpu_destroy(shygpu_model *m) {
 // A cluster shape is used only after the occupancy query says that at least
 // one such cluster fits the device (clusters above 8 CTAs need the
 // non-portable attribute set first).
-static int check_cluster_shape(int CL, int threads, size_t smem) {
-  cudaError_t e = zeta_kernel_setup(CL, smem);
-  if (e != cudaSuccess) return fail(SHY_EARG, "cluster size %d / %zu B shared memory not available: %s", CL, smem, cudaGetErrorString(e));
-  int n = zeta_max_active_clusters(CL, threads, smem);
-  if (n < 1) return fail(SHY_EARG, "a cluster of %d CTAs x %d threads (%zu B shared) does not fit the device", CL, threads, smem);
+static int check_cluster_shape(int CL, int threads) {
+  cudaError_t e = zeta_kernel_setup(CL);
+  if (e != cudaSuccess) return fail(SHY_EARG, "cluster size %d not available: %s", CL, cudaGetErrorString(e));
+  int n = zeta_max_active_clusters(CL, threads);
+  if (n < 1) return fail(SHY_EARG, "a cluster of %d CTAs x %d threads does not fit the device", CL, threads);
   return SHY_OK;
 }
 
@@ -1256,8 +1326,8 @@ extern "C" int shygpu_create(int32_t nbasin, const shy_basin *B, const shy_param
       A.alloc(&d.val32, nnz + 4) || A.alloc(&d.dinv32, NKN) || A.alloc(&d.r32, NKN) ||
       A.alloc(&d.p32, NKN) || A.alloc(&d.q32, NKN) || A.alloc(&d.z32, NKN) ||
       A.alloc(&d.e32, NKN) || A.alloc(&d.s32, NKN) || A.alloc(&d.t32, NKN) ||
-      A.alloc(&d.rh32, NKN) || A.alloc(&d.v32, NKN) || A.alloc(&d.cg4[0], NKN) ||
-      A.alloc(&d.cg4[1], NKN) || A.alloc(&d.cg2, NKN + 2) || A.alloc(&d.hia, (size_t)12 * NEL) || A.alloc(&d.unv, NEL) || A.alloc(&d.vnv, NEL) ||
+      A.alloc(&d.rh32, NKN) || A.alloc(&d.v32, NKN) ||
+      A.alloc(&d.hia, (size_t)12 * NEL) || A.alloc(&d.unv, NEL) || A.alloc(&d.vnv, NEL) ||
       A.alloc(&d.usv, EL) || A.alloc(&d.vsv, EL) ||
       A.alloc(&d.wl, (size_t)NKN * (NLV + 1)) || A.alloc(&d.rho, NL) || A.alloc(&d.ddx, EL) ||
       A.alloc(&d.ddxi, m->cor ? EL : 1) || A.alloc(&d.cbnd, NSC) || A.alloc(&d.vol_node, NKN) || A.alloc(&d.vbud_node, NKN) ||
@@ -1284,6 +1354,12 @@ extern "C" int shygpu_create(int32_t nbasin, const shy_basin *B, const shy_param
   if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess)
     return bail(fail(SHY_ECUDA, "stream creation failed"));
   // zeta solver launch shape: one cluster per basin, about 2k rows per CTA
+  m->xy_h.resize((size_t)2 * NKN);
+  for (int b = 0, k = 0; b < nbasin; b++)
+    for (int i = 0; i < B[b].nkn; i++, k++) {
+      m->xy_h[(size_t)2 * k] = B[b].xgv[i];
+      m->xy_h[(size_t)2 * k + 1] = B[b].ygv[i];
+    }
   m->rowptr_h = rowptr;
   m->col_h = col;
   if (cudaEventCreateWithFlags(&m->ev_fork, cudaEventDisableTiming) != cudaSuccess)
@@ -1332,8 +1408,8 @@ extern "C" int shygpu_set_option(shygpu_model *m, const char *name, double value
     }
   }
   else if (n == "zeta_variant") {
-    // 0: vectors in global memory; 1: shared memory when every basin fits a
-    // cluster, else the device-wide solver; 2: the device-wide solver
+    // 0: clusters with vectors in global memory; 1, 2: one device-wide launch,
+    // the resident solver when every basin fits it, else the streaming one
     if (iv < 0 || iv > 2) return fail(SHY_EARG, "zeta_variant: 0, 1 or 2");
     m->zvariant = iv;
     ST_TRY(build_zeta_plan(m, m->zforce_CL, m->zforce_threads));
@@ -1404,7 +1480,7 @@ extern "C" double shygpu_get_option(shygpu_model *m, const char *name) {
   if (n == "inner_tol_frac") return m->tol_frac;
   if (n == "max_outer") return m->max_outer;
   if (n == "symmetric") return m->sym;
-  if (n == "zeta_variant") return m->zcl.empty() ? -1 : (m->zcl[0].grid ? 2 : (m->zcl[0].sm ? 1 : 0));
+  if (n == "zeta_variant") return m->zcl.empty() ? -1 : (m->zcl[0].grid || m->zcl[0].team ? 2 : 0);
   if (n == "zeta_grid_ctas") return m->zcl.empty() ? -1 : m->zcl[0].G;
   if (n == "zeta_stage") return m->zcl.empty() || !m->zcl[0].grid ? m->zstage : (m->zcl[0].staged ? 1 : 0);
   if (n == "zeta_tile_rows") return m->ztile_rows > 0 ? m->ztile_rows : zeta_grid_tile_rows();
@@ -2703,7 +2779,6 @@ extern "C" int shygpu_autotune(shygpu_model *m, int32_t steps, char *choice, int
       groups.push_back({
           {{"zeta_stage", 0}, {"zeta_tile_rows", 1024}, {"zeta_variant", 1}},
           {{"zeta_stage", 0}, {"zeta_tile_rows", 512}, {"zeta_variant", 2}},
-          {{"zeta_stage", 0}, {"zeta_tile_rows", 1024}, {"zeta_variant", 2}},
           {{"zeta_stage", 0}, {"zeta_tile_rows", 2048}, {"zeta_variant", 2}},
           {{"zeta_stage", 1}, {"zeta_tile_rows", 1024}, {"zeta_variant", 2}},
           {{"zeta_stage", 0}, {"zeta_tile_rows", 1024}, {"zeta_variant", 0}},
@@ -3051,7 +3126,7 @@ static int simsys_solve_impl(int n, const float *z) {
   za.explicit_mode = g_sys.explicit_mode; za.inner_rtol = 1e-4f; za.max_outer = 12; za.sym = 0;
   int CL = n >= 16384 ? 8 : (n >= 4096 ? 4 : (n >= 1024 ? 2 : 1));
   int threads = n >= 4096 ? 1024 : 512;
-  ST_TRY(check_cluster_shape(CL, threads, 0));
+  ST_TRY(check_cluster_shape(CL, threads));
   za.blist = g_sys.d_blist0;
   cudaError_t e = launch_zeta(d, za, CL, threads, 1, st);
   if (e != cudaSuccess) return fail(SHY_ECUDA, "system_solve launch: %s", cudaGetErrorString(e));

@@ -6,7 +6,7 @@
 // that each has about the same rows and a basin's tiles spread over many
 // CTAs, so the work of the few basins still iterating late in a solve is
 // shared out.
-// The solver is the one of k_zeta_sm (system_solve,
+// The solver is the one of k_zeta_team (system_solve,
 // sparskit_admin.f90:115-334, with the reference's stop test
 // ||r|| <= rtol*||r0|| + atol, spk_iters.f90:3304-3360): FP64 residual
 // refinement around Jacobi-preconditioned Chronopoulos-Gear CG in FP32, the
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(NT, STAGED ? 1 : 2) k_zeta_grid(Dev d, ZetaArg
       while (iq < ntl && !staged_stage(gs[s_tile[iq].w].stage)) iq++;
       if (iq < ntl) {
         const int4 tl = s_tile[iq];
-        stage_issue<C16>(gp, SL, sbuf[b], mbar[b], tl.x, tl.y, d.cg4[gs[tl.w].cur]);
+        stage_issue<C16>(gp, SL, sbuf[b], mbar[b], tl.x, tl.y, gp.cg4[gs[tl.w].cur]);
         iq++;
       }
     };
@@ -454,8 +454,8 @@ __global__ void __launch_bounds__(NT, STAGED ? 1 : 2) k_zeta_grid(Dev d, ZetaArg
         const unsigned char *buf = dsm + 128 + (size_t)b * SL.bytes;
         const float4 *sq = reinterpret_cast<const float4 *>(buf + SL.q4);
         const float *sev = reinterpret_cast<const float *>(buf + SL.ev) + (a - (a & ~3));
-        const float4 *qi = d.cg4[g.cur];
-        float4 *qo = d.cg4[g.cur ^ 1];
+        const float4 *qi = gp.cg4[g.cur];
+        float4 *qo = gp.cg4[g.cur ^ 1];
         const int R = e - a;
         const float fa = stage == G_ITER ? (float)g.alpha : 0.f;
         const float fb = stage == G_ITER ? (float)g.beta : 0.f;
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(NT, STAGED ? 1 : 2) k_zeta_grid(Dev d, ZetaArg
         // the FP64 residual t (its norm is the stop test's), the scaled S t
         // the FP32 sweep starts from, a zero correction; the first pass of
         // a solve also writes the scaled off-diagonal entries of its rows
-        float4 *qo = d.cg4[g.cur];
+        float4 *qo = gp.cg4[g.cur];
         const bool scale = g.first != 0;
         for (int i = a + tid; i < e; i += nth) {
           const double t = grid_resid_row(d, i);
@@ -505,8 +505,8 @@ __global__ void __launch_bounds__(NT, STAGED ? 1 : 2) k_zeta_grid(Dev d, ZetaArg
         for (int i = a + tid; i < e; i += nth) d.x64[i] = 2. * (double)za.zguess[i] - (double)za.zprev[i];
       } else if (stage == G_SPMV0) {
         // w = (S A S) r (fa = fb = 0 leave r); p = s = 0
-        const float4 *qi = d.cg4[g.cur];
-        float4 *qo = d.cg4[g.cur ^ 1];
+        const float4 *qi = gp.cg4[g.cur];
+        float4 *qo = gp.cg4[g.cur ^ 1];
         for (int i = a + tid; i < e; i += nth) {
           const float4 me = qi[i];
           const float w = grid_spmv_row<C16>(gp, i, qi, 0.f, 0.f, me.x);
@@ -518,8 +518,8 @@ __global__ void __launch_bounds__(NT, STAGED ? 1 : 2) k_zeta_grid(Dev d, ZetaArg
       } else if (stage == G_ITER) {
         // p = r + b p, s = w + b s, e += a p, r -= a s, w = (S A S) r
         const float fa = (float)g.alpha, fb = (float)g.beta;
-        const float4 *qi = d.cg4[g.cur];
-        float4 *qo = d.cg4[g.cur ^ 1];
+        const float4 *qi = gp.cg4[g.cur];
+        float4 *qo = gp.cg4[g.cur ^ 1];
         for (int i = a + tid; i < e; i += nth) {
           const float4 me = qi[i];
           const float p = me.x + fb * me.w;

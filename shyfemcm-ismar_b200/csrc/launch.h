@@ -72,22 +72,6 @@ void launch_nh(const Dev &d, const NhSys &s, int which, cudaStream_t st);
 cudaError_t launch_nh_solve(const CsrGrid &a, int G, cudaStream_t st);
 int nh_solve_capacity();           // CTAs of k_nh_solve that fit the device at once
 
-// shape of the shared-memory zeta solver: CL CTAs of `threads` per basin,
-// rows per CTA (capacity) and nonzeros per CTA (capacity), dynamic smem
-struct ZetaShape {
-  int CL = 0, threads = 0, chunk = 0, nnzcap = 0, halocap = 0;
-  size_t smem = 0;
-};
-
-// maps of the shared-memory zeta solver for one cluster shape:
-// loc[s]  -- local shared-memory column index of CSR slot s (own rows first,
-//            then the CTA's halo slots)
-// push    -- for each row (push_ptr[i]..push_ptr[i+1]) the halo slots of other
-//            CTAs that hold a copy of it, packed (rank << 24) | slot
-struct ZetaMaps {
-  const int *loc = nullptr, *push_ptr = nullptr, *push = nullptr;
-};
-
 // the device-wide zeta solver (k_zeta_grid).  Each basin's rows are cut into
 // tiles of a fixed row count (the last one shorter); tile t = {row0, row1,
 // basin, slot} is worked by one CTA (cptr/clist), where `slot` indexes the CTA's table
@@ -118,10 +102,47 @@ struct GridPlan {
   float *xval = nullptr;
   int nx = 0;
   float *sd = nullptr, *ecor = nullptr;
+  float4 *cg4[2] = {nullptr, nullptr};   // {r, w = S A S r, s, p} per row, two generations
   double *partial = nullptr;       // [2][ntile][4] partial sums of the tiles
   unsigned *ctr = nullptr;         // [8]: barrier arrivals, 3 active counts, abort flag, release
   unsigned phantom = 0;            // arrivals the barrier waits for beyond its CTAs (0; 1 in the timeout test)
   long long spin_limit = 0;        // polls before a barrier wait gives up
+};
+
+// widest team of the resident solver (k_zeta_team) whose members read each
+// other's sums, and the words of a slot that carries a member's
+constexpr int kTeamAllToAll = 128, kTeamSlotWords = 8;
+
+// one CTA's share of a basin in the resident solver: rows rows[row0 ..
+// row0+nrow), ghost copies ghost[ghost0 ..+nghost); rank of T members,
+// whose sums sit in slots slot0 .. slot0+T-1
+struct TeamMember {
+  int basin, T, rank, slot0;
+  int row0, nrow, ghost0, nghost;
+};
+
+// the resident zeta solver.  Member m is worked by one CTA (cptr/clist, in
+// one order of the basins common to all CTAs).  Per row of the shares, in
+// their order: the global row (sign bit: some other member holds a ghost of
+// it), the place of the diagonal among the row's CSR slots with the count
+// of the others (dpos: place | count << 8), and the share's local column
+// (own rows, from zeta_team_rows() on the ghosts) of the first eight off-diagonal entries (lcol, as
+// byte offsets into a float array; the row itself on padding); rows with more keep the rest in a tail (tptr,
+// tcol, tslot, tval; null when no row has one).  word: four exchange buffers
+// of one word per row; part: two buffers of a
+// slot per member and the phantom, for its own sums and for the totals.
+struct TeamPlan {
+  const TeamMember *mem = nullptr;
+  const int *cptr = nullptr, *clist = nullptr;
+  const int *rows = nullptr, *dpos = nullptr, *ghost = nullptr;
+  const unsigned short *lcol = nullptr, *tcol = nullptr;
+  const int *tptr = nullptr, *tslot = nullptr;
+  float *tval = nullptr;
+  unsigned long long *word = nullptr, *part = nullptr;
+  unsigned *ctr = nullptr, *cta_cnt = nullptr;   // abort word; launches made, per CTA
+  int nslot = 0;                   // the last one the phantom's
+  int phantom = 0;                 // 1: every exchange waits for a member that does not exist (timeout test)
+  long long spin_limit = 0;        // polls before a wait gives up
 };
 
 // a group of basins solved by one launch with one cluster shape
@@ -131,21 +152,26 @@ struct ZetaClass {
   int G = 0;                       // its CTAs
   size_t gsmem = 0;                // its dynamic shared memory
   GridPlan gp;
-  bool sm = false;                 // shared-memory variant (else global memory)
+  bool team = false;               // resident cooperative variant (all basins, one launch)
+  TeamPlan tp;
   int CL = 1, threads = 512;
-  ZetaShape zs;                    // capacities of the shared-memory variant
   std::vector<int> basins;
   int *d_blist = nullptr;          // device copy of basins
 };
 
 // nb clusters of CL CTAs; cluster c solves basin za.blist[c]
 cudaError_t launch_zeta(const Dev &d, const ZetaArgs &za, int CL, int threads, int nb, cudaStream_t st);
-cudaError_t launch_zeta_sm(const Dev &d, const ZetaArgs &za, const ZetaShape &zs, const ZetaMaps &zm,
-                           int nb, cudaStream_t st);
 // the device-wide variant: G CTAs, cooperative; clears gp.ctr first.  staged:
 // the TMA-staged form with `smem` bytes of dynamic shared memory
 cudaError_t launch_zeta_grid(const Dev &d, const ZetaArgs &za, const GridPlan &gp, int G, bool staged,
                              size_t smem, cudaStream_t st);
+// the resident variant: G CTAs, cooperative
+cudaError_t launch_zeta_team(const Dev &d, const ZetaArgs &za, const TeamPlan &tp, int G, cudaStream_t st);
+int zeta_team_capacity();    // its CTAs that fit the device at once (0 on error)
+int zeta_team_rows();        // rows a CTA holds at most
+int zeta_team_share(int nk); // rows a CTA gets at most in a basin of nk rows
+int zeta_team_ghosts();      // ghost rows a CTA holds
+long long zeta_team_spin_limit();
 // CTAs of k_zeta_grid that fit the device at once (0 on error)
 int zeta_grid_capacity(bool staged, size_t smem);
 // dynamic shared memory of the staged form (16-bit or absolute columns)
@@ -154,8 +180,7 @@ int zeta_grid_max_slots();   // basins one CTA can hold
 int zeta_grid_max_tiles();   // tiles one CTA can hold
 int zeta_grid_tile_rows();   // rows per tile
 long long zeta_grid_spin_limit();   // default barrier poll limit
-// smem > 0 prepares the shared-memory variant for that many dynamic bytes
-cudaError_t zeta_kernel_setup(int CL, size_t smem);
-int zeta_max_active_clusters(int CL, int threads, size_t smem);
+cudaError_t zeta_kernel_setup(int CL);
+int zeta_max_active_clusters(int CL, int threads);
 
 }  // namespace shy

@@ -1,5 +1,5 @@
 // step_zeta.cu -- launch wrappers and set-up of the zeta solvers (k_zeta,
-// k_zeta_sm, k_zeta_grid).  See step.cu.
+// k_zeta_team, k_zeta_grid).  See step.cu.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -14,15 +14,15 @@
 #include "k_zeta.cuh"
 #include "k_zeta_global.cuh"
 #include "k_zeta_grid.cuh"
+#include "k_zeta_team.cuh"
 
 namespace shy {
 
-static cudaLaunchConfig_t zeta_config(int CL, int threads, int nclusters, size_t smem, cudaStream_t st,
+static cudaLaunchConfig_t zeta_config(int CL, int threads, int nclusters, cudaStream_t st,
                                       cudaLaunchAttribute *attr) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nclusters * CL, 1, 1);
   cfg.blockDim = dim3(threads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = CL;
@@ -35,15 +35,8 @@ static cudaLaunchConfig_t zeta_config(int CL, int threads, int nclusters, size_t
 
 cudaError_t launch_zeta(const Dev &d, const ZetaArgs &za, int CL, int threads, int nb, cudaStream_t st) {
   cudaLaunchAttribute attr[1];
-  cudaLaunchConfig_t cfg = zeta_config(CL, threads, nb, 0, st, attr);
+  cudaLaunchConfig_t cfg = zeta_config(CL, threads, nb, st, attr);
   return cudaLaunchKernelEx(&cfg, k_zeta, d, za, CL);
-}
-
-cudaError_t launch_zeta_sm(const Dev &d, const ZetaArgs &za, const ZetaShape &zs, const ZetaMaps &zm,
-                           int nb, cudaStream_t st) {
-  cudaLaunchAttribute attr[1];
-  cudaLaunchConfig_t cfg = zeta_config(zs.CL, zs.threads, nb, zs.smem, st, attr);
-  return cudaLaunchKernelEx(&cfg, k_zeta_sm, d, za, zs, zm);
 }
 
 cudaError_t launch_zeta_grid(const Dev &d, const ZetaArgs &za, const GridPlan &gp, int G, bool staged,
@@ -66,6 +59,42 @@ cudaError_t launch_zeta_grid(const Dev &d, const ZetaArgs &za, const GridPlan &g
   return c16 ? cudaLaunchKernelEx(&cfg, k_zeta_grid<512, false, true>, d, za, gp)
              : cudaLaunchKernelEx(&cfg, k_zeta_grid<512, false, false>, d, za, gp);
 }
+
+constexpr int kTeamNT = 512, kTeamR = 4, kTeamGR = 1;
+constexpr long long kTeamSpinLimit = 1LL << 22;   // polls of a word: seconds
+
+cudaError_t launch_zeta_team(const Dev &d, const ZetaArgs &za, const TeamPlan &tp, int G, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3(G, 1, 1);
+  cfg.blockDim = dim3(kTeamNT, 1, 1);
+  cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_zeta_team<kTeamNT, kTeamR, kTeamGR>, d, za, tp);
+}
+
+int zeta_team_capacity() {
+  int dev = 0, nsm = 0, nb = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_zeta_team<kTeamNT, kTeamR, kTeamGR>, kTeamNT, 0) !=
+      cudaSuccess)
+    return 0;
+  return std::min(nb * nsm, kTeamNT);      // one thread polls each member of a team
+}
+int zeta_team_rows() { return kTeamNT * kTeamR; }
+// Rows a CTA gets: 1024 in basins of up to 40 shares, where a team's
+// latency matters (7k rows: 0.31 ms a solve on 7 CTAs, 0.38 ms on 4), 2048
+// in larger ones, where more members only make the exchange slower (250k
+// rows: 0.42 ms on 123, 0.66 ms on 245) and the ensemble's basins take turns
+// on the CTAs (64 basins: 2.8 ms against 3.2 ms).  It depends on the basin
+// alone, so that its bits do.
+int zeta_team_share(int nk) { return nk <= 40960 ? kTeamNT * kTeamR / 2 : kTeamNT * kTeamR; }
+int zeta_team_ghosts() { return kTeamNT * kTeamGR; }
+long long zeta_team_spin_limit() { return kTeamSpinLimit; }
 
 size_t zeta_grid_stage_smem(bool c16) { return 128 + 2 * (size_t)stage_layout(c16 ? 16 : 32).bytes; }
 
@@ -100,23 +129,15 @@ int zeta_grid_max_tiles() { return kGridMaxTiles; }
 int zeta_grid_tile_rows() { return kGridTileRows; }
 long long zeta_grid_spin_limit() { return kGridSpinLimit; }
 
-cudaError_t zeta_kernel_setup(int CL, size_t smem) {
-  cudaError_t e = cudaSuccess;
-  if (CL > 8) {
-    e = cudaFuncSetAttribute(k_zeta, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_zeta_sm, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  }
-  if (e == cudaSuccess && smem > 0)
-    e = cudaFuncSetAttribute(k_zeta_sm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  return e;
+cudaError_t zeta_kernel_setup(int CL) {
+  return CL > 8 ? cudaFuncSetAttribute(k_zeta, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) : cudaSuccess;
 }
 
-int zeta_max_active_clusters(int CL, int threads, size_t smem) {
+int zeta_max_active_clusters(int CL, int threads) {
   cudaLaunchAttribute attr[1];
-  cudaLaunchConfig_t cfg = zeta_config(CL, threads, 1, smem, nullptr, attr);
+  cudaLaunchConfig_t cfg = zeta_config(CL, threads, 1, nullptr, attr);
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, smem > 0 ? (const void *)k_zeta_sm : (const void *)k_zeta, &cfg) != cudaSuccess)
-    return -1;
+  if (cudaOccupancyMaxActiveClusters(&n, (const void *)k_zeta, &cfg) != cudaSuccess) return -1;
   return n;
 }
 
