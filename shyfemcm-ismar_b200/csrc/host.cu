@@ -343,11 +343,11 @@ static void drop_graphs(shygpu_model *m) {
 
 static int check_cluster_shape(int CL, int threads);
 
-// Zeta launch plan.  A symmetric model runs in one cooperative launch over
-// the device: the resident solver (k_zeta_team), or the streaming one
-// (k_zeta_grid) when a basin does not fit on chip or its tiles are asked
-// for.  Other systems run k_zeta, a cluster per basin with vectors in global
-// memory, in one launch per cluster size on streams of their own.
+// Zeta launch plan.  A model runs in one cooperative launch over the device:
+// the resident solver (k_zeta_team), or, when a basin does not fit on chip
+// or its tiles are asked for, the streaming one (k_zeta_grid) if the system
+// is symmetric.  The rest runs k_zeta, a cluster per basin with vectors in
+// global memory, in one launch per cluster size on streams of their own.
 static void free_zeta_plan(shygpu_model *m) {
   for (ZetaClass &c : m->zcl) {
     if (c.d_blist) cudaFree(c.d_blist);
@@ -532,29 +532,87 @@ static int build_grid_class(shygpu_model *m) {
   return SHY_OK;
 }
 
-// nodes ord[lo, hi) cut into T compact patches of nearly equal size by
-// recursive bisection of their coordinates, across the longer side; patch r
-// of the T holds ord[cut[r], cut[r+1])
-static void bisect_nodes(std::vector<int> &ord, const float *xy, int lo, int hi, int r, int T, std::vector<int> &cut) {
+// a row with its place in the plane
+struct PlaneRow { float x[2]; int i; };
+
+// rows v[0, n) cut into T compact patches of nearly equal size by recursive
+// bisection, across the longer side; patch r holds v[cut[r], cut[r+1]),
+// rows in order (gathers of neighbours stay local); `at` is v's place
+static void bisect_rows(PlaneRow *v, int n, int at, int r, int T, int *cut) {
   if (T == 1) {
-    cut[r] = lo;
-    std::sort(ord.begin() + lo, ord.begin() + hi);   // rows in order: gathers of neighbours stay local
+    cut[r] = at;
+    std::sort(v, v + n, [](const PlaneRow &p, const PlaneRow &q) { return p.i < q.i; });
     return;
   }
   float a[2] = {INFINITY, INFINITY}, b[2] = {-INFINITY, -INFINITY};
-  for (int i = lo; i < hi; i++)
-    for (int c = 0; c < 2; c++) {
-      a[c] = std::min(a[c], xy[2 * (size_t)ord[i] + c]);
-      b[c] = std::max(b[c], xy[2 * (size_t)ord[i] + c]);
-    }
+  for (int i = 0; i < n; i++)
+    for (int c = 0; c < 2; c++) { a[c] = std::min(a[c], v[i].x[c]); b[c] = std::max(b[c], v[i].x[c]); }
   const int c = b[1] - a[1] > b[0] - a[0] ? 1 : 0;
-  const int T1 = T / 2, mid = lo + (int)((long long)(hi - lo) * T1 / T);
-  std::nth_element(ord.begin() + lo, ord.begin() + mid, ord.begin() + hi, [&](int p, int q) {
-    const float u = xy[2 * (size_t)p + c], v = xy[2 * (size_t)q + c];
-    return u != v ? u < v : p < q;
+  const int T1 = T / 2, mid = (int)((long long)n * T1 / T);
+  std::nth_element(v, v + mid, v + n, [c](const PlaneRow &p, const PlaneRow &q) {
+    return p.x[c] != q.x[c] ? p.x[c] < q.x[c] : p.i < q.i;
   });
-  bisect_nodes(ord, xy, lo, mid, r, T1, cut);
-  bisect_nodes(ord, xy, mid, hi, r + T1, T - T1, cut);
+  bisect_rows(v, mid, at, r, T1, cut);
+  bisect_rows(v + mid, n - mid, at + mid, r + T1, T - T1, cut);
+}
+
+// what the resident solver needs to know of one basin (rows k0 .. k0+nk-1)
+struct TeamBasin {
+  std::vector<int> cut;                            // first row of each share, and nk
+  std::vector<int> ghost, gptr;                    // ghosts of the shares, offsets
+  std::vector<int> tcount, tslot;                  // rows' tail lengths, tail slots
+  std::vector<unsigned short> tcol;
+  std::vector<int> rows, dpos;
+  std::vector<unsigned short> lcol;                // K columns a row
+  int most = 0;                                    // most ghosts of a share
+};
+
+// shares of the rows k0 .. k0+nk-1 of the CSR pattern with coordinates xy:
+// TR: ghosts' first place in a share; K: entries of a row's block
+static void team_basin(const int *rowptr, const int *col, const float *xy, int k0, int nk, int T, int TR, int K,
+                       TeamBasin &B) {
+  std::vector<PlaneRow> v(nk);
+  for (int j = 0; j < nk; j++) v[j] = PlaneRow{{xy[2 * (size_t)(k0 + j)], xy[2 * (size_t)(k0 + j) + 1]}, k0 + j};
+  B.cut.assign(T + 1, nk);
+  bisect_rows(v.data(), nk, 0, 0, T, B.cut.data());
+  std::vector<int> own(nk), place(nk), seen(nk, -1), gplace(nk), gl;
+  std::vector<char> sent(nk, 0);
+  for (int r = 0; r < T; r++)
+    for (int j = B.cut[r]; j < B.cut[r + 1]; j++) { own[v[j].i - k0] = r; place[v[j].i - k0] = j - B.cut[r]; }
+  B.rows.resize(nk);
+  B.dpos.resize(nk);
+  B.lcol.resize((size_t)K * nk);
+  B.tcount.assign(nk, 0);
+  B.gptr.assign(1, 0);
+  for (int r = 0; r < T; r++) {
+    gl.clear();
+    for (int j = B.cut[r]; j < B.cut[r + 1]; j++)
+      for (int s = rowptr[v[j].i]; s < rowptr[v[j].i + 1]; s++) {
+        const int c = col[s] - k0;
+        if (own[c] != r && seen[c] != r) { seen[c] = r; gl.push_back(c); sent[c] = 1; }
+      }
+    std::sort(gl.begin(), gl.end());
+    B.most = std::max(B.most, (int)gl.size());
+    for (size_t g = 0; g < gl.size(); g++) { gplace[gl[g]] = TR + (int)g; B.ghost.push_back(k0 + gl[g]); }
+    B.gptr.push_back((int)B.ghost.size());
+    if (B.most > zeta_team_ghosts()) return;       // refused by the caller
+    for (int j = B.cut[r]; j < B.cut[r + 1]; j++) {
+      const int i = v[j].i, s0 = rowptr[i];
+      unsigned short *lc = &B.lcol[(size_t)K * j];
+      int n = 0, dp = 0;
+      for (int s = s0; s < rowptr[i + 1]; s++) {
+        const int c = col[s] - k0;
+        if (c == i - k0) { dp = s - s0; continue; }
+        const int l = own[c] == r ? place[c] : gplace[c];
+        if (n < K) lc[n] = (unsigned short)(4 * l);
+        else { B.tcol.push_back((unsigned short)l); B.tslot.push_back(s); B.tcount[j]++; }
+        n++;
+      }
+      for (int k = n; k < K; k++) lc[k] = (unsigned short)(4 * (j - B.cut[r]));
+      B.dpos[j] = dp | n << 8;
+    }
+  }
+  for (int j = 0; j < nk; j++) B.rows[j] = v[j].i | (sent[v[j].i - k0] ? (int)0x80000000u : 0);
 }
 
 // The resident class: every basin in one cooperative launch of k_zeta_team.
@@ -565,69 +623,55 @@ static void bisect_nodes(std::vector<int> &ord, const float *xy, int lo, int hi,
 // needs more CTAs than are resident or a share has more ghosts than a CTA
 // holds.
 static int build_team_class(shygpu_model *m) {
-  const int cap = zeta_team_capacity(), TR = zeta_team_rows(), NKN = m->NKN;
+  const int cap = zeta_team_capacity(), TR = zeta_team_rows(), NKN = m->NKN, NB = m->nbasin;
+  constexpr int K = 8;
   if (cap < 1) return fail(SHY_ECUDA, "zeta resident solver: no resident CTA fits the device");
-  std::vector<TeamMember> mem;
-  std::vector<int> ord(NKN), cut, first(m->nbasin + 1, 0);
-  for (int i = 0; i < NKN; i++) ord[i] = i;
+  std::vector<int> width(NB);
   long long ctas = 0;
-  for (int b = 0; b < m->nbasin; b++) {
-    const BasinPar &bp = m->par[b];
-    const int rows = zeta_team_share(bp.nk), T = (bp.nk + rows - 1) / rows;
-    if (T > cap) return fail(SHY_EARG, "zeta resident solver: basin %d needs %d CTAs, %d are resident", b, T, cap);
-    cut.assign(T + 1, bp.k0 + bp.nk);
-    bisect_nodes(ord, m->xy_h.data(), bp.k0, bp.k0 + bp.nk, 0, T, cut);
-    const int slot0 = (int)mem.size();
-    for (int r = 0; r < T; r++) mem.push_back(TeamMember{b, T, r, slot0, cut[r], cut[r + 1] - cut[r], 0, 0});
+  for (int b = 0; b < NB; b++) {
+    const int nk = m->par[b].nk, rows = zeta_team_share(nk);
+    width[b] = (nk + rows - 1) / rows;
+    if (width[b] > cap)
+      return fail(SHY_EARG, "zeta resident solver: basin %d needs %d CTAs, %d are resident", b, width[b], cap);
+    ctas += width[b];
+  }
+  // the basins' shares, on the host's cores
+  std::vector<TeamBasin> tb(NB);
+  {
+    std::atomic<int> next{0};
+    auto work = [&] {
+      for (int b; (b = next++) < NB;)
+        team_basin(m->rowptr_h.data(), m->col_h.data(), m->xy_h.data(), m->par[b].k0, m->par[b].nk, width[b], TR, K, tb[b]);
+    };
+    const int nt = NKN < 100000 ? 1 : std::min(NB, std::max(1, std::min(8, (int)std::thread::hardware_concurrency())));
+    std::vector<std::thread> pool;
+    for (int t = 1; t < nt; t++) pool.emplace_back(work);
+    work();
+    for (std::thread &t : pool) t.join();
+  }
+  std::vector<TeamMember> mem;
+  std::vector<int> first(NB + 1, 0), ord, dpos, ghost, tptr(1, 0), tslot;
+  std::vector<unsigned short> lcol, tcol;
+  ord.reserve(NKN); dpos.reserve(NKN); lcol.reserve((size_t)K * NKN); tptr.reserve(NKN + 1);
+  for (int b = 0; b < NB; b++) {
+    TeamBasin &B = tb[b];
+    if (B.most > zeta_team_ghosts())
+      return fail(SHY_EARG, "zeta resident solver: a share of basin %d has %d ghosts", b, B.most);
+    const int slot0 = (int)mem.size(), row0 = (int)ord.size(), g0 = (int)ghost.size();
+    for (int r = 0; r < width[b]; r++)
+      mem.push_back(TeamMember{b, width[b], r, slot0, row0 + B.cut[r], B.cut[r + 1] - B.cut[r], g0 + B.gptr[r],
+                               B.gptr[r + 1] - B.gptr[r]});
     first[b + 1] = (int)mem.size();
-    ctas += T;
+    ord.insert(ord.end(), B.rows.begin(), B.rows.end());
+    dpos.insert(dpos.end(), B.dpos.begin(), B.dpos.end());
+    lcol.insert(lcol.end(), B.lcol.begin(), B.lcol.end());
+    ghost.insert(ghost.end(), B.ghost.begin(), B.ghost.end());
+    for (int n : B.tcount) tptr.push_back(tptr.back() + n);
+    tslot.insert(tslot.end(), B.tslot.begin(), B.tslot.end());
+    tcol.insert(tcol.end(), B.tcol.begin(), B.tcol.end());
+    B = TeamBasin();
   }
-  // shares: ghosts in row order, local columns, tails
-  std::vector<int> dpos(NKN), ghost, local(NKN), own(NKN), seen(NKN, -1), tptr, tslot;
-  std::vector<unsigned short> lcol((size_t)8 * NKN), tcol;
-  std::vector<char> sent(NKN, 0);
-  for (size_t q = 0; q < mem.size(); q++)
-    for (int j = 0; j < mem[q].nrow; j++) { own[ord[mem[q].row0 + j]] = (int)q; local[ord[mem[q].row0 + j]] = j; }
-  bool tail = false;
-  for (int i = 0; i < NKN && !tail; i++) tail = m->rowptr_h[i + 1] - m->rowptr_h[i] > 9;
-  if (tail) tptr.assign(NKN + 1, 0);
-  std::vector<int> gidx(NKN, 0), gl;
-  for (size_t q = 0; q < mem.size(); q++) {
-    TeamMember &M = mem[q];
-    gl.clear();
-    for (int j = 0; j < M.nrow; j++) {
-      const int i = ord[M.row0 + j];
-      for (int s = m->rowptr_h[i]; s < m->rowptr_h[i + 1]; s++) {
-        const int c = m->col_h[s];
-        if (own[c] != (int)q && seen[c] != (int)q) { seen[c] = (int)q; gl.push_back(c); sent[c] = 1; }
-      }
-    }
-    if ((int)gl.size() > zeta_team_ghosts())
-      return fail(SHY_EARG, "zeta resident solver: a share of %d rows has %d ghosts", M.nrow, (int)gl.size());
-    std::sort(gl.begin(), gl.end());
-    M.ghost0 = (int)ghost.size();
-    M.nghost = (int)gl.size();
-    for (size_t g = 0; g < gl.size(); g++) gidx[gl[g]] = TR + (int)g;
-    ghost.insert(ghost.end(), gl.begin(), gl.end());
-    for (int j = 0; j < M.nrow; j++) {
-      const int i = ord[M.row0 + j], s0 = m->rowptr_h[i];
-      unsigned short *lc = &lcol[(size_t)8 * (M.row0 + j)];
-      int n = 0, dp = 0;
-      for (int s = s0; s < m->rowptr_h[i + 1]; s++) {
-        const int c = m->col_h[s];
-        if (c == i) { dp = s - s0; continue; }
-        const int l = own[c] == (int)q ? local[c] : gidx[c];
-        if (n < 8) lc[n] = (unsigned short)(4 * l);
-        else { tcol.push_back((unsigned short)l); tslot.push_back(s); }
-        n++;
-      }
-      for (int k = n; k < 8; k++) lc[k] = (unsigned short)(4 * j);
-      dpos[M.row0 + j] = dp | n << 8;
-      if (tail) tptr[M.row0 + j + 1] = (int)tcol.size();
-    }
-  }
-  for (int &i : ord)
-    if (sent[i]) i |= (int)0x80000000u;
+  const bool tail = !tslot.empty();
   // teams to CTAs
   const int G = (int)std::min<long long>(cap, ctas);
   std::vector<int> job(m->nbasin);
@@ -710,13 +754,13 @@ static int build_zeta_plan(shygpu_model *m, int forceCL, int forceThreads) {
 static int build_zeta_plan_impl(shygpu_model *m, int forceCL, int forceThreads) {
   free_zeta_plan(m);
   const int NKN = m->NKN;
-  // symmetric systems (zeta_variant 1 and 2): the resident solver where every
-  // basin fits it, else, or when its tiles are asked for, the streaming
-  // device-wide solver
-  if (m->sym && m->zvariant && forceCL <= 0) {
+  // zeta_variant 1 and 2: the resident solver where every basin fits it, else,
+  // or when its tiles are asked for, the streaming device-wide solver for
+  // symmetric systems
+  if (m->zvariant && forceCL <= 0) {
     int st = SHY_EARG;
-    if (!m->zstage && (m->ztile_rows == 0 || m->ztile_rows == zeta_grid_tile_rows())) st = build_team_class(m);
-    if (st == SHY_EARG) {
+    if (!m->sym || (!m->zstage && (m->ztile_rows == 0 || m->ztile_rows == zeta_grid_tile_rows()))) st = build_team_class(m);
+    if (st == SHY_EARG && m->sym) {
       free_zeta_plan(m);
       st = build_grid_class(m);
     }

@@ -101,13 +101,14 @@ struct TeamShared {
   float u[NT * R + NT * GR];       // the product's input: own rows, from NT * R on the ghosts
   float sd[NT * R + NT * GR];      // Jacobi scale D^-1/2
   double x[NT * R + NT * GR];      // the FP64 iterate
-  double wred[4][NT / 32];         // sums of the warps
+  double wred[6][NT / 32];         // sums of the warps
   double tot[4];                   // sums of the team
-  double tsum[4][NT / 32];         // its members', a warp's worth each
+  double tsum[6][NT / 32];         // its members', a warp's worth each
   double resid0, tol, rn, rn2, rs2;   // ||r0||, the target, ||r||, ||r||^2, ||S r||^2
   double itol2;                    // an FP32 sweep's target for ||S r||^2
   double rgamma, ralpha;           // 1 / gamma, 1 / alpha of the last update
-  float fa, fb;                    // alpha, beta of the next one
+  double rho, alpha;               // BiCGStab's (rh, r) and alpha
+  float fa, fb, fo;                // alpha, beta, omega of the next update
   int stop, ok;
   TeamMember M;
 };
@@ -242,7 +243,11 @@ __device__ __forceinline__ u64 *team_buf(const TeamPlan &tp, const Dev &d, unsig
   return tp.word + (size_t)(xi & 1u) * d.NKN;
 }
 
-template <int NT, int R, int GR>
+// SYM: CG on the symmetrically scaled system S A S; else BiCGStab (van der
+// Vorst 1992) on A D^-1 (right Jacobi preconditioning), for systems with
+// Coriolis or dry elements, and the repeat loop of wetting and drying
+// (hydrodynamic.f90:374-404).  Both scaled matrices have a unit diagonal.
+template <int NT, int R, int GR, bool SYM>
 __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPlan tp) {
   typedef TeamShared<NT, R, GR> SH;
   __shared__ SH sh;
@@ -265,13 +270,53 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
     unsigned xi = 0u;                            // exchanges of this solve
     auto number = [&] { return (launch << 16) | (xi & 0xffffu); };
     const int n = M.nrow, nr = (n + NT - 1) / NT;   // rows, rows a thread at most
+    const int echunk = (P.ne + M.T - 1) / M.T;   // this member's elements (wetting and drying)
+    const int ea = P.e0 + min(P.ne, M.rank * echunk), eb = min(P.e0 + P.ne, ea + echunk);
     if (M.rank == 0 && tid < kMaxScal) O.stab[tid] = 0.f;   // reset for k_stab's max
     const float dtf = (float)P.dt;
-    const bool extrap = za.zprev != nullptr && O.steps > 0;
+    // wetting and drying: a domain that can change with the solution
+    const bool wd = !SYM && wd_basin(P) && !za.explicit_mode;
+    const bool extrap = za.zprev != nullptr && O.steps > 0 && !wd;
+    // a barrier of the team that also makes its global writes visible; sums
+    // one value
+    auto team_barrier = [&](double &v) -> bool {
+      __threadfence();
+      const double y = warp_sum2(v, 0.);
+      if ((tid & 15) == 0) sh.wred[(tid >> 4) & 1][tid >> 5] = y;
+      __syncthreads();
+      double tot[2];
+      const bool k = team_totals<1, NT>(sh, tp, M, number(), xi, abortv, tot);
+      if (tid == 0) sh.tot[0] = tot[0];
+      if (!k) sh.ok = 0;
+      __syncthreads();
+      __threadfence();
+      xi++;
+      v = sh.tot[0];
+      return sh.ok != 0;
+    };
+    int iters = 0, outer = 0, refine = 0;
+    for (int rep = 0;; rep++) {
+    if (wd) {
+      bool fine = true;
+      double none = 0.;
+      for (int j = tid; j < n; j += NT) fine &= wd_setnod(d, tp.rows[M.row0 + j] & 0x7fffffff);
+      if (!fine) set_status(&O, SHY_EDEPTH);     // the open boundary dried (setnod :245)
+      if (!team_barrier(none)) { dead = true; break; }
+      for (int e = ea + tid; e < eb; e += NT)
+        if (__ldcg(&d.iweg[e]) != 0) wd_dry_system(d, e);
+      if (!team_barrier(none)) { dead = true; break; }
+    }
+    // the guess: the old level, in repeats the last solution
+    const float *guess = rep == 0 ? za.zguess : d.zn;
+    auto level = [&](int i) { return (double)(wd ? __ldcg(guess + i) : guess[i]); };
 
     // ---- assembly (FP64 sums in element order), Jacobi scale, and the
     // residuals of both starts, the old level's (the stop test's r0) and the
     // extrapolated one's ----
+    auto elem = [&](const float *a, int c, int e) {   // dry systems are written in this launch
+      const float *q = a + (size_t)c * za.cs + (size_t)e * za.es;
+      return wd ? __ldcg(q) : *q;
+    };
     int ri[R];                                   // global row, sign bit: published
     float rsA[R], rsB[R];
     double v4[4] = {0., 0., 0., 0.};
@@ -294,15 +339,17 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
         for (int k = 0; k < 8; k++) {
           const bool in = p0 + k < p1;
           const int e3 = in ? d.inc[p0 + k] : 0, e = e3 / 3, ii = e3 - 3 * e;
-          ha[k] = in ? za.hia[(size_t)(4 * ii) * za.cs + (size_t)e * za.es] : 0.f;
-          hb[k] = in ? za.hik[(size_t)ii * za.cs + (size_t)e * za.es] : 0.f;
+          ha[k] = in ? elem(za.hia, 4 * ii, e) : 0.f;
+          hb[k] = in ? elem(za.hik, ii, e) : 0.f;
         }
 #pragma unroll
         for (int k = 0; k < 8; k++) { diag += (double)ha[k]; rhs += (double)hb[k]; }
       }
-      rhs += (double)(dtf * d.rqv[i]);
+      // adjust_mass_flux (bnd_routines.f90:1185-1210): no flux enters a node
+      // out of the system
+      if (!(wd && d.inod[i] == -2)) rhs += (double)(dtf * d.rqv[i]);
       d.rhs64[i] = rhs;
-      const double zg = (double)za.zguess[i];
+      const double zg = level(i);
       if (za.explicit_mode) {
         const double x0 = diag != 0. ? rhs / diag : 0.;
         d.x64[i] = x0;
@@ -318,25 +365,25 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
         const int q0s = d.slot_ptr[sl], q1s = d.slot_ptr[sl + 1];
         const int srcA = d.slot_src[q0s], srcB = q1s - q0s > 1 ? d.slot_src[q0s + 1] : -1;
         const int eA = srcA / 9, eB = srcB < 0 ? 0 : srcB / 9;
-        double a = (double)za.hia[(size_t)(srcA - 9 * eA) * za.cs + (size_t)eA * za.es];
-        if (srcB >= 0) a += (double)za.hia[(size_t)(srcB - 9 * eB) * za.cs + (size_t)eB * za.es];
+        double a = (double)elem(za.hia, srcA - 9 * eA, eA);
+        if (srcB >= 0) a += (double)elem(za.hia, srcB - 9 * eB, eB);
         for (int t = q0s + 2; t < q1s; t++) {
           const int e = d.slot_src[t] / 9;
-          a += (double)za.hia[(size_t)(d.slot_src[t] - 9 * e) * za.cs + (size_t)e * za.es];
+          a += (double)elem(za.hia, d.slot_src[t] - 9 * e, e);
         }
         const int c = d.col[sl];
         d.val64[sl] = a;
-        tA -= a * (double)za.zguess[c];
-        if (extrap) tB -= a * (2. * (double)za.zguess[c] - (double)za.zprev[c]);
+        tA -= a * level(c);
+        if (extrap) tB -= a * (2. * level(c) - (double)za.zprev[c]);
       };
 #pragma unroll
       for (int k = 0; k < 8; k++)
         if (k < nd) entry(k);
       for (int k = 8; k < nd; k++) entry(k);
-      const float sd = diag > 0. ? (float)(1. / sqrt(diag)) : 1.f;
+      const float sd = SYM ? (diag > 0. ? (float)(1. / sqrt(diag)) : 1.f) : (diag != 0. ? (float)(1. / diag) : 1.f);
       sh.sd[j] = sd;
-      rsA[r] = (float)((double)sd * tA);
-      rsB[r] = (float)((double)sd * tB);
+      rsA[r] = (float)(SYM ? (double)sd * tA : tA);
+      rsB[r] = (float)(SYM ? (double)sd * tB : tB);
       v4[0] += tA * tA;
       v4[1] += (double)rsA[r] * rsA[r];
       v4[2] += tB * tB;
@@ -344,15 +391,15 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
     }
     if (za.explicit_mode) {                      // system_set_explicit: no coupling between rows
       if (M.rank == 0 && tid == 0) { O.iters = 0; O.refinements = 0; O.resid0 = 0.; O.resid = 0.; }
-      continue;
+      break;
     }
     unsigned ep = number();
 #pragma unroll
     for (int r = 0; r < R; r++)
       if (ri[r] < 0) {
         const size_t i = (size_t)(ri[r] & 0x7fffffff);
-        word_put(tp.word + i, __float_as_uint(sh.sd[r * NT + tid]), ep);
-        word_put(tp.word + (size_t)d.NKN + i, 0u, ep);   // every launch renews every word
+        word_put(team_buf(tp, d, xi) + i, __float_as_uint(sh.sd[r * NT + tid]), ep);
+        if (rep == 0) word_put(team_buf(tp, d, xi + 1u) + i, 0u, ep);   // every launch renews every word
         word_put(tp.word + 2 * (size_t)d.NKN + i, __float_as_uint(rsA[r]), ep);
         word_put(tp.word + 3 * (size_t)d.NKN + i, __float_as_uint(rsB[r]), ep);
       }
@@ -376,7 +423,7 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
       if (jg < M.nghost) {
         gi[g] = tp.ghost[M.ghost0 + jg];
         const u64 *p = tp.word + gi[g];
-        const u64 *const pw[3] = {p, p + 2 * (size_t)d.NKN, p + 3 * (size_t)d.NKN};
+        const u64 *const pw[3] = {team_buf(tp, d, xi) + gi[g], p + 2 * (size_t)d.NKN, p + 3 * (size_t)d.NKN};
         unsigned h[3];
         ok = words_wait(tp, pw, ep, abortv, h) && ok;
         sd = __uint_as_float(h[0]);
@@ -389,13 +436,14 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
       double tot[4];
       ok = team_totals<2, NT>(sh, tp, M, ep, xi, abortv, tot) && ok;
       if (tid == 0) {
-        sh.resid0 = sqrt(tot[0]);
-        sh.tol = (double)P.rtol * sh.resid0 + (double)P.atol;
-        const bool useB = extrap && sh.resid0 > sh.tol;
+        const double rA = sqrt(tot[0]);
+        if (rep == 0) sh.resid0 = rA;
+        sh.tol = (double)P.rtol * rA + (double)P.atol;
+        const bool useB = extrap && rA > sh.tol;
         sh.stop = useB;
         sh.rn2 = useB ? tot[2] : tot[0];
         sh.rs2 = useB ? tot[3] : tot[1];
-        sh.rn = useB ? sqrt(tot[2]) : sh.resid0;
+        sh.rn = useB ? sqrt(tot[2]) : rA;
       }
     }
     if (!ok) sh.ok = 0;
@@ -407,7 +455,7 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
     float rr[R];
     {
       const bool useB = sh.stop != 0;
-      auto start = [&](int i) { return useB ? 2. * (double)za.zguess[i] - (double)za.zprev[i] : (double)za.zguess[i]; };
+      auto start = [&](int i) { return useB ? 2. * level(i) - (double)za.zprev[i] : level(i); };
 #pragma unroll
       for (int r = 0; r < R; r++) {
         const int j = r * NT + tid;
@@ -434,7 +482,7 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
       col[r][0] = c4.x; col[r][1] = c4.y; col[r][2] = c4.z; col[r][3] = c4.w;
       const int i = ri[r] & 0x7fffffff;
       const int dn = tp.dpos[M.row0 + j], dp = dn & 0xff, nd = dn >> 8;
-      const double sdi = (double)sh.sd[j];
+      const double sdi = SYM ? (double)sh.sd[j] : 1.;
       const double *a = d.val64 + d.rowptr[i];
 #pragma unroll
       for (int k = 0; k < 8; k++)
@@ -445,10 +493,12 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
           tp.tval[t] = (float)(d.val64[tp.tslot[t]] * sdi * (double)sh.sd[tp.tcol[t]]);
     }
 
-    auto product = [&](float (&w)[R]) {          // (S A S) u of the own rows: unit diagonal, then slot order
+    // the scaled matrix times u for the own rows: the unit diagonal times
+    // their own input x, then slot order
+    auto product = [&](const float (&x)[R], float (&w)[R]) {
 #pragma unroll
       for (int r = 0; r < R; r++) {
-        w[r] = rr[r];
+        w[r] = x[r];
         if (r >= nr) continue;
 #pragma unroll
         for (int k = 0; k < 8; k++)
@@ -458,20 +508,24 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
             w[r] += tp.tval[t] * sh.u[tp.tcol[t]];
       }
     };
-    // Publish a value per bordering row and two sums, receive the ghosts' and
+    // Publish a value per bordering row and the sums v, receive the ghosts' and
     // the totals, which thread 0 hands to `post`; the CTA barrier at the end
     // makes what it stores in sh visible.
-    auto exchange = [&](const float (&w)[R], float (&gw)[GR], double va, double vb, auto post) -> bool {
+    auto exchange = [&](const float (&w)[R], float (&gw)[GR], const auto &v, auto post) -> bool {
+      constexpr int NP = sizeof(v) / (2 * sizeof(double));
       ep = number();
       u64 *buf = team_buf(tp, d, xi);
 #pragma unroll
       for (int r = 0; r < R; r++)
         if (ri[r] < 0) word_put(buf + (ri[r] & 0x7fffffff), __float_as_uint(w[r]), ep);
-      const double y = warp_sum2(va, vb);
-      if ((tid & 15) == 0) sh.wred[(tid >> 4) & 1][tid >> 5] = y;
+#pragma unroll
+      for (int c = 0; c < NP; c++) {
+        const double y = warp_sum2(v[2 * c], v[2 * c + 1]);
+        if ((tid & 15) == 0) sh.wred[2 * c + ((tid >> 4) & 1)][tid >> 5] = y;
+      }
       __syncthreads();
-      double tot[2];
-      bool k = team_totals<1, NT>(sh, tp, M, ep, xi, abortv, tot);
+      double tot[2 * NP];
+      bool k = team_totals<NP, NT>(sh, tp, M, ep, xi, abortv, tot);
       if (tid == 0) post(tot);
 #pragma unroll
       for (int g = 0; g < GR; g++) {
@@ -486,72 +540,160 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
       return sh.ok != 0;
     };
 
-    int iters = 0, outer = 0;
-    for (;;) {
+    for (outer = 0;;) {
       if (sh.rn <= sh.tol || outer >= za.max_outer) break;
       if (tid == 0) {
-        // the FP32 sweep's target, moved into the norm of the scaled residual
+        // the FP32 sweep's target, moved into the norm of the residual it works on
         const double it0 = fmax((double)za.inner_rtol * sh.rn, tfrac(za) * sh.tol);
         sh.itol2 = sh.rn2 > 0. ? it0 * it0 * (sh.rs2 / sh.rn2) : 0.;
       }
-      float p[R], s[R], e[R], w[R], gp[GR], gs[GR], ge[GR], gw[GR];
+      float e[R], ge[GR];                        // the correction
 #pragma unroll
-      for (int r = 0; r < R; r++) {
-        p[r] = s[r] = e[r] = 0.f;
-        sh.u[r * NT + tid] = rr[r];
-      }
+      for (int r = 0; r < R; r++) e[r] = 0.f;
 #pragma unroll
-      for (int g = 0; g < GR; g++) {
-        gp[g] = gs[g] = ge[g] = 0.f;
-        sh.u[NT * R + g * NT + gtid] = gr[g];
-      }
-      __syncthreads();
-      product(w);
-      double va = 0., vb = 0.;
-#pragma unroll
-      for (int r = 0; r < R; r++) { va += (double)rr[r] * rr[r]; vb += (double)w[r] * rr[r]; }
-      // 1 / gamma and 1 / alpha are kept, so that beta = g / gamma and alpha
-      // = g / (delta - beta g / alpha) wait for one division
-      if (!exchange(w, gw, va, vb, [&](const double (&t)[2]) {
-            sh.fa = (float)(t[0] / t[1]);
-            sh.fb = 0.f;
-            sh.rgamma = 1. / t[0];
-            sh.ralpha = t[1] * sh.rgamma;
-          })) { dead = true; break; }
-      for (int inner = 1;; inner++) {
-        // p = r + b p, s = w + b s, e += a p, r -= a s, then w = (S A S) r
-        const float fa = sh.fa, fb = sh.fb;
+      for (int g = 0; g < GR; g++) ge[g] = 0.f;
+      if constexpr (SYM) {
+        float p[R], s[R], w[R], gp[GR], gs[GR], gw[GR];
 #pragma unroll
         for (int r = 0; r < R; r++) {
-          p[r] = rr[r] + fb * p[r];
-          s[r] = w[r] + fb * s[r];
-          e[r] += fa * p[r];
-          rr[r] -= fa * s[r];
+          p[r] = s[r] = 0.f;
           sh.u[r * NT + tid] = rr[r];
         }
 #pragma unroll
         for (int g = 0; g < GR; g++) {
-          gp[g] = gr[g] + fb * gp[g];
-          gs[g] = gw[g] + fb * gs[g];
-          ge[g] += fa * gp[g];
-          gr[g] -= fa * gs[g];
+          gp[g] = gs[g] = 0.f;
           sh.u[NT * R + g * NT + gtid] = gr[g];
         }
         __syncthreads();
-        product(w);
-        va = vb = 0.;
+        product(rr, w);
+        double v[2] = {0., 0.};
 #pragma unroll
-        for (int r = 0; r < R; r++) { va += (double)rr[r] * rr[r]; vb += (double)w[r] * rr[r]; }
-        if (!exchange(w, gw, va, vb, [&](const double (&t)[2]) {
-              const double beta = t[0] * sh.rgamma, den = t[1] - beta * t[0] * sh.ralpha;
-              sh.fa = (float)(t[0] / den);
-              sh.fb = (float)beta;
-              sh.stop = !(t[0] > sh.itol2) || !(t[0] == t[0]) || inner >= P.maxit;
+        for (int r = 0; r < R; r++) { v[0] += (double)rr[r] * rr[r]; v[1] += (double)w[r] * rr[r]; }
+        // 1 / gamma and 1 / alpha are kept, so that beta = g / gamma and alpha
+        // = g / (delta - beta g / alpha) wait for one division
+        if (!exchange(w, gw, v, [&](const double (&t)[2]) {
+              sh.fa = (float)(t[0] / t[1]);
+              sh.fb = 0.f;
               sh.rgamma = 1. / t[0];
-              sh.ralpha = den * sh.rgamma;
+              sh.ralpha = t[1] * sh.rgamma;
             })) { dead = true; break; }
-        iters++;
-        if (sh.stop) break;
+        for (int inner = 1;; inner++) {
+          // p = r + b p, s = w + b s, e += a p, r -= a s, then w = (S A S) r
+          const float fa = sh.fa, fb = sh.fb;
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            p[r] = rr[r] + fb * p[r];
+            s[r] = w[r] + fb * s[r];
+            e[r] += fa * p[r];
+            rr[r] -= fa * s[r];
+            sh.u[r * NT + tid] = rr[r];
+          }
+#pragma unroll
+          for (int g = 0; g < GR; g++) {
+            gp[g] = gr[g] + fb * gp[g];
+            gs[g] = gw[g] + fb * gs[g];
+            ge[g] += fa * gp[g];
+            gr[g] -= fa * gs[g];
+            sh.u[NT * R + g * NT + gtid] = gr[g];
+          }
+          __syncthreads();
+          product(rr, w);
+          v[0] = v[1] = 0.;
+#pragma unroll
+          for (int r = 0; r < R; r++) { v[0] += (double)rr[r] * rr[r]; v[1] += (double)w[r] * rr[r]; }
+          if (!exchange(w, gw, v, [&](const double (&t)[2]) {
+                const double beta = t[0] * sh.rgamma, den = t[1] - beta * t[0] * sh.ralpha;
+                sh.fa = (float)(t[0] / den);
+                sh.fb = (float)beta;
+                sh.stop = !(t[0] > sh.itol2) || !(t[0] == t[0]) || inner >= P.maxit;
+                sh.rgamma = 1. / t[0];
+                sh.ralpha = den * sh.rgamma;
+              })) { dead = true; break; }
+          iters++;
+          if (sh.stop) break;
+        }
+      } else {
+        // p = r + beta (p - omega v), v = A p, alpha = rho / (rh v),
+        // s = r - alpha v, t = A s, omega = (t s) / (t t), r = s - omega t.
+        // rho of the next turn and ||r||^2 follow from the sums of s and t, so
+        // an iteration takes two exchanges.
+        float rh[R], p[R], q[R], w[R], gp[GR], gv[GR], gw[GR];
+#pragma unroll
+        for (int r = 0; r < R; r++) { rh[r] = rr[r]; p[r] = q[r] = 0.f; }
+#pragma unroll
+        for (int g = 0; g < GR; g++) gp[g] = gv[g] = 0.f;
+        if (tid == 0) {
+          sh.rho = sh.rs2;                       // (rh, r)
+          sh.fb = sh.fo = 0.f;
+        }
+        __syncthreads();
+        for (int inner = 1;; inner++) {
+          const float fb = sh.fb, fo = sh.fo;    // beta, omega
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            p[r] = rr[r] + fb * (p[r] - fo * q[r]);
+            sh.u[r * NT + tid] = p[r];
+          }
+#pragma unroll
+          for (int g = 0; g < GR; g++) {
+            gp[g] = gr[g] + fb * (gp[g] - fo * gv[g]);
+            sh.u[NT * R + g * NT + gtid] = gp[g];
+          }
+          __syncthreads();
+          product(p, q);
+          double v1[2] = {0., 0.};
+#pragma unroll
+          for (int r = 0; r < R; r++) v1[0] += (double)rh[r] * q[r];
+          if (!exchange(q, gv, v1, [&](const double (&t)[2]) {
+                sh.alpha = t[0] != 0. ? sh.rho / t[0] : 0.;
+                sh.fa = (float)sh.alpha;
+              })) { dead = true; break; }
+          const float fa = sh.fa;
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            rr[r] -= fa * q[r];                  // s
+            sh.u[r * NT + tid] = rr[r];
+          }
+#pragma unroll
+          for (int g = 0; g < GR; g++) {
+            gr[g] -= fa * gv[g];
+            sh.u[NT * R + g * NT + gtid] = gr[g];
+          }
+          __syncthreads();
+          product(rr, w);                        // t
+          double v[6] = {0., 0., 0., 0., 0., 0.};
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            const double sd = rr[r], td = w[r], hd = rh[r];
+            v[0] += td * sd;
+            v[1] += td * td;
+            v[2] += sd * sd;
+            v[3] += hd * sd;
+            v[4] += hd * td;
+          }
+          if (!exchange(w, gw, v, [&](const double (&t)[6]) {
+                const double om = t[1] > 0. ? t[0] / t[1] : 0.;
+                const double rho = t[3] - om * t[4], r2 = t[2] - om * (2. * t[0] - om * t[1]);
+                sh.fo = (float)om;
+                sh.fb = (float)((rho / sh.rho) * (sh.alpha / om));
+                sh.stop = !(r2 > sh.itol2) || !(r2 == r2) || om == 0. || sh.alpha == 0. || rho == 0. ||
+                          inner >= P.maxit;
+                sh.rho = rho;
+              })) { dead = true; break; }
+          const float fw = sh.fo;
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            e[r] += fa * p[r] + fw * rr[r];
+            rr[r] -= fw * w[r];
+          }
+#pragma unroll
+          for (int g = 0; g < GR; g++) {
+            ge[g] += fa * gp[g] + fw * gr[g];
+            gr[g] -= fw * gw[g];
+          }
+          iters++;
+          if (sh.stop) break;
+        }
       }
       if (dead) break;
       // the correction in FP64, and the residual it leaves
@@ -566,7 +708,7 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
         }
       outer++;
       __syncthreads();
-      va = vb = 0.;
+      double v[2] = {0., 0.};
 #pragma unroll
       for (int r = 0; r < R; r++) {
         const int j = r * NT + tid;
@@ -582,23 +724,39 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
         if (tp.tptr)
           for (int q2 = tp.tptr[M.row0 + j]; q2 < tp.tptr[M.row0 + j + 1]; q2++)
             t -= d.val64[tp.tslot[q2]] * sh.x[tp.tcol[q2]];
-        rr[r] = (float)((double)sh.sd[j] * t);
-        va += t * t;
-        vb += (double)rr[r] * rr[r];
+        rr[r] = (float)(SYM ? (double)sh.sd[j] * t : t);
+        v[0] += t * t;
+        v[1] += (double)rr[r] * rr[r];
       }
-      if (!exchange(rr, gr, va, vb, [&](const double (&t)[2]) {
+      if (!exchange(rr, gr, v, [&](const double (&t)[2]) {
             sh.rn2 = t[0];
             sh.rs2 = t[1];
             sh.rn = sqrt(t[0]);
           })) { dead = true; break; }
     }
     if (dead) break;
+    refine += outer;
 #pragma unroll
     for (int r = 0; r < R; r++)
       if (r * NT + tid < n) d.zn[ri[r] & 0x7fffffff] = (float)sh.x[r * NT + tid];
+    if (!wd) break;
+    // setweg(1): elements with a vertex below hzmin leave; then the step
+    // counters, every element on the first pass of the step (a new time)
+    double none = 0., chg = 0.;
+    if (!team_barrier(none)) { dead = true; break; }   // the new levels of every row
+    for (int e = ea + tid; e < eb; e += NT) {
+      chg += wd_take_away(d, P, e) ? 1. : 0.;
+      d.iwet[e] = wd_count(d.iweg[e], d.iwet[e], rep == 0);
+    }
+    if (!team_barrier(chg)) { dead = true; break; }
+    if (chg == 0.) break;
+    if (rep + 1 >= kWetDryRepeats) { if (M.rank == 0 && tid == 0) set_status(&O, SHY_ENOCONV); break; }
+    }
+    if (dead) break;
+    if (za.explicit_mode) continue;
     if (tid == 0 && M.rank == 0) {
       O.iters = iters;
-      O.refinements = outer;
+      O.refinements = refine;
       O.resid0 = sh.resid0;
       O.resid = sh.rn;
       if (!(sh.rn <= sh.tol)) set_status(&O, SHY_ENOCONV);

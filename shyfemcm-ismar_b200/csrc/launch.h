@@ -111,7 +111,7 @@ struct GridPlan {
 
 // widest team of the resident solver (k_zeta_team) whose members read each
 // other's sums, and the words of a slot that carries a member's
-constexpr int kTeamAllToAll = 128, kTeamSlotWords = 8;
+constexpr int kTeamAllToAll = 128, kTeamSlotWords = 16;
 
 // one CTA's share of a basin in the resident solver: rows rows[row0 ..
 // row0+nrow), ghost copies ghost[ghost0 ..+nghost); rank of T members,

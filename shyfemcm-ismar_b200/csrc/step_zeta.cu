@@ -73,17 +73,20 @@ cudaError_t launch_zeta_team(const Dev &d, const ZetaArgs &za, const TeamPlan &t
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_zeta_team<kTeamNT, kTeamR, kTeamGR>, d, za, tp);
+  return za.sym ? cudaLaunchKernelEx(&cfg, k_zeta_team<kTeamNT, kTeamR, kTeamGR, true>, d, za, tp)
+                : cudaLaunchKernelEx(&cfg, k_zeta_team<kTeamNT, kTeamR, kTeamGR, false>, d, za, tp);
 }
 
 int zeta_team_capacity() {
-  int dev = 0, nsm = 0, nb = 0;
+  int dev = 0, nsm = 0, na = 0, nb = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_zeta_team<kTeamNT, kTeamR, kTeamGR>, kTeamNT, 0) !=
-      cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&na, k_zeta_team<kTeamNT, kTeamR, kTeamGR, true>, kTeamNT, 0) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_zeta_team<kTeamNT, kTeamR, kTeamGR, false>, kTeamNT, 0) !=
+          cudaSuccess)
     return 0;
-  return std::min(nb * nsm, kTeamNT);      // one thread polls each member of a team
+  return std::min(std::min(na, nb) * nsm, kTeamNT);      // one thread polls each member of a team
 }
 int zeta_team_rows() { return kTeamNT * kTeamR; }
 // Rows a CTA gets: 1024 in basins of up to 40 shares, where a team's

@@ -44,6 +44,35 @@ def test_resident_solver_matches_streaming(nx, ny):
     assert np.abs(za - zb).max() <= TOL
 
 
+@pytest.mark.parametrize("nx,ny", [(3, 3), (57, 9), (41, 25), (205, 40), (257, 160)])
+def test_resident_bicgstab_matches_clusters(nx, ny):
+    """Coriolis: the non-symmetric system, against the cluster solver."""
+    case = basin(nx, ny)
+    case["fcorv"] = np.full(case["nel"], 1.0e-4, np.float32)
+    (za,), a = levels(case)
+    (zb,), b = levels(case, zeta_variant=0)
+    assert a.get_option("zeta_variant") == 2 and b.get_option("zeta_variant") == 0
+    assert np.abs(za - zb).max() <= TOL
+
+
+@pytest.mark.parametrize("nx,ny", [(33, 9), (161, 33)])
+def test_resident_wetting_and_drying_matches_clusters(nx, ny):
+    """The repeat loop inside one CTA and inside a team: the same dry
+    elements and vertex levels as the cluster solver's."""
+    case = cases.flat_case(nx=nx, ny=ny, lx=200.0 * (nx - 1), ly=200.0 * (ny - 1))
+    out = []
+    for variant in (1, 0):
+        m = shygpu.Model(case)
+        m.set_option("zeta_variant", variant)
+        m.set_state(0)
+        m.run(30)
+        out.append((m.wetdry(0), m.get_state(0)["zenv"]))
+    assert (out[0][0][0] != 0).any()
+    for a, b in zip(out[0][0], out[1][0]):
+        assert np.array_equal(a, b)
+    assert np.abs(out[0][1] - out[1][1]).max() <= TOL
+
+
 def test_basin_keeps_its_bits_in_a_batch():
     cs = [basin(57, 9, 1), basin(205, 40, 2), basin(3, 3, 3), basin(300, 150, 4)]
     batch, _ = levels(cs)
