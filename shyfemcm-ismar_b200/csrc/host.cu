@@ -273,6 +273,8 @@ struct shygpu_model {
   CsrGrid nhg;                       // the solver's work arrays
   std::vector<int2> nh_rows;         // per basin its rows [x, y) (empty range: hydrostatic)
   int nh_G = 0;                      // CTAs of the solver's launch at most
+  TeamPlan nh_team;                  // the resident solver's plan of it, nh_TG CTAs (0: it does not fit)
+  int nh_TG = 0;
   std::vector<BasinPar> par;
   std::vector<int> nlv_b;
   Arena arena;
@@ -348,17 +350,15 @@ static int check_cluster_shape(int CL, int threads);
 // or its tiles are asked for, the streaming one (k_zeta_grid) if the system
 // is symmetric.  The rest runs k_zeta, a cluster per basin with vectors in
 // global memory, in one launch per cluster size on streams of their own.
+static void free_team_plan(TeamPlan &t) {
+  cudaFree(t.base);
+  t = TeamPlan();
+}
+
 static void free_zeta_plan(shygpu_model *m) {
   for (ZetaClass &c : m->zcl) {
     if (c.d_blist) cudaFree(c.d_blist);
-    if (c.team) {
-      const TeamPlan &t = c.tp;
-      for (const void *p : {(const void *)t.mem, (const void *)t.cptr, (const void *)t.clist, (const void *)t.rows,
-                            (const void *)t.dpos, (const void *)t.ghost, (const void *)t.lcol, (const void *)t.tcol,
-                            (const void *)t.tptr, (const void *)t.tslot, (const void *)t.tval, (const void *)t.word,
-                            (const void *)t.part, (const void *)t.ctr, (const void *)t.cta_cnt})
-        cudaFree((void *)p);
-    }
+    if (c.team) free_team_plan(c.tp);
     if (c.grid) {
       cudaFree((void *)c.gp.tile); cudaFree((void *)c.gp.btile); cudaFree((void *)c.gp.cslot);
       cudaFree((void *)c.gp.cnslot); cudaFree((void *)c.gp.cowner);
@@ -567,10 +567,10 @@ struct TeamBasin {
   int most = 0;                                    // most ghosts of a share
 };
 
-// shares of the rows k0 .. k0+nk-1 of the CSR pattern with coordinates xy:
-// TR: ghosts' first place in a share; K: entries of a row's block
-static void team_basin(const int *rowptr, const int *col, const float *xy, int k0, int nk, int T, int TR, int K,
+// shares of the rows k0 .. k0+nk-1 of the CSR pattern with coordinates xy
+static void team_basin(const int *rowptr, const int *col, const float *xy, int k0, int nk, int T, const TeamShape &sh,
                        TeamBasin &B) {
+  const int K = sh.entries;
   std::vector<PlaneRow> v(nk);
   for (int j = 0; j < nk; j++) v[j] = PlaneRow{{xy[2 * (size_t)(k0 + j)], xy[2 * (size_t)(k0 + j) + 1]}, k0 + j};
   B.cut.assign(T + 1, nk);
@@ -593,9 +593,9 @@ static void team_basin(const int *rowptr, const int *col, const float *xy, int k
       }
     std::sort(gl.begin(), gl.end());
     B.most = std::max(B.most, (int)gl.size());
-    for (size_t g = 0; g < gl.size(); g++) { gplace[gl[g]] = TR + (int)g; B.ghost.push_back(k0 + gl[g]); }
+    for (size_t g = 0; g < gl.size(); g++) { gplace[gl[g]] = sh.rows + (int)g; B.ghost.push_back(k0 + gl[g]); }
     B.gptr.push_back((int)B.ghost.size());
-    if (B.most > zeta_team_ghosts()) return;       // refused by the caller
+    if (B.most > sh.ghosts) return;       // refused by the caller
     for (int j = B.cut[r]; j < B.cut[r + 1]; j++) {
       const int i = v[j].i, s0 = rowptr[i];
       unsigned short *lc = &B.lcol[(size_t)K * j];
@@ -615,51 +615,53 @@ static void team_basin(const int *rowptr, const int *col, const float *xy, int k
   for (int j = 0; j < nk; j++) B.rows[j] = v[j].i | (sent[v[j].i - k0] ? (int)0x80000000u : 0);
 }
 
-// The resident class: every basin in one cooperative launch of k_zeta_team.
-// A basin's team has as many CTAs as its rows need (so its shares and sums
-// depend on it alone); teams are dealt to the CTAs widest first, each to the
-// CTAs that are free soonest, in one order common to all CTAs (so no two
-// CTAs wait for each other's later work).  Returns SHY_EARG when a basin
-// needs more CTAs than are resident or a share has more ghosts than a CTA
-// holds.
-static int build_team_class(shygpu_model *m) {
-  const int cap = zeta_team_capacity(), TR = zeta_team_rows(), NKN = m->NKN, NB = m->nbasin;
-  constexpr int K = 8;
-  if (cap < 1) return fail(SHY_ECUDA, "zeta resident solver: no resident CTA fits the device");
-  std::vector<int> width(NB);
-  long long ctas = 0;
-  for (int b = 0; b < NB; b++) {
-    const int nk = m->par[b].nk, rows = zeta_team_share(nk);
-    width[b] = (nk + rows - 1) / rows;
-    if (width[b] > cap)
-      return fail(SHY_EARG, "zeta resident solver: basin %d needs %d CTAs, %d are resident", b, width[b], cap);
-    ctas += width[b];
+// one system of a resident plan: its basin, rows k0 .. k0+nk-1, CTAs
+struct TeamJob { int basin, k0, nk, width; };
+
+// The plan of the resident solver for the systems `jobs` of one CSR pattern
+// with coordinates xy per row.  A team has as many CTAs as its rows need (so
+// its shares and sums depend on it alone); teams are dealt to the CTAs widest
+// first, each to the CTAs that are free soonest, in one order common to all
+// CTAs (so no two CTAs wait for each other's later work).  Returns SHY_EARG
+// when a system needs more CTAs than are resident or a share has more ghosts
+// than a CTA holds.
+static int make_team_plan(TeamPlan &t, int &G, const TeamShape &sh, const std::vector<int> &rowptr,
+                          const std::vector<int> &col, const std::vector<float> &xy, const std::vector<TeamJob> &jobs,
+                          bool bar_test) {
+  const int NB = (int)jobs.size(), K = sh.entries;
+  if (sh.capacity < 1) return fail(SHY_ECUDA, "resident solver: no resident CTA fits the device");
+  long long ctas = 0, nrows = 0;
+  for (const TeamJob &j : jobs) {
+    if (j.width > sh.capacity)
+      return fail(SHY_EARG, "resident solver: basin %d needs %d CTAs, %d are resident", j.basin, j.width, sh.capacity);
+    ctas += j.width;
+    nrows += j.nk;
   }
-  // the basins' shares, on the host's cores
+  // the systems' shares, on the host's cores
   std::vector<TeamBasin> tb(NB);
   {
     std::atomic<int> next{0};
     auto work = [&] {
       for (int b; (b = next++) < NB;)
-        team_basin(m->rowptr_h.data(), m->col_h.data(), m->xy_h.data(), m->par[b].k0, m->par[b].nk, width[b], TR, K, tb[b]);
+        team_basin(rowptr.data(), col.data(), xy.data(), jobs[b].k0, jobs[b].nk, jobs[b].width, sh, tb[b]);
     };
-    const int nt = NKN < 100000 ? 1 : std::min(NB, std::max(1, std::min(8, (int)std::thread::hardware_concurrency())));
+    const int nt = nrows < 100000 ? 1 : std::min(NB, std::max(1, std::min(8, (int)std::thread::hardware_concurrency())));
     std::vector<std::thread> pool;
-    for (int t = 1; t < nt; t++) pool.emplace_back(work);
+    for (int q = 1; q < nt; q++) pool.emplace_back(work);
     work();
-    for (std::thread &t : pool) t.join();
+    for (std::thread &q : pool) q.join();
   }
   std::vector<TeamMember> mem;
   std::vector<int> first(NB + 1, 0), ord, dpos, ghost, tptr(1, 0), tslot;
   std::vector<unsigned short> lcol, tcol;
-  ord.reserve(NKN); dpos.reserve(NKN); lcol.reserve((size_t)K * NKN); tptr.reserve(NKN + 1);
+  ord.reserve(nrows); dpos.reserve(nrows); lcol.reserve((size_t)K * nrows); tptr.reserve(nrows + 1);
   for (int b = 0; b < NB; b++) {
     TeamBasin &B = tb[b];
-    if (B.most > zeta_team_ghosts())
-      return fail(SHY_EARG, "zeta resident solver: a share of basin %d has %d ghosts", b, B.most);
+    if (B.most > sh.ghosts)
+      return fail(SHY_EARG, "resident solver: a share of basin %d has %d ghosts", jobs[b].basin, B.most);
     const int slot0 = (int)mem.size(), row0 = (int)ord.size(), g0 = (int)ghost.size();
-    for (int r = 0; r < width[b]; r++)
-      mem.push_back(TeamMember{b, width[b], r, slot0, row0 + B.cut[r], B.cut[r + 1] - B.cut[r], g0 + B.gptr[r],
+    for (int r = 0; r < jobs[b].width; r++)
+      mem.push_back(TeamMember{jobs[b].basin, jobs[b].width, r, slot0, row0 + B.cut[r], B.cut[r + 1] - B.cut[r], g0 + B.gptr[r],
                                B.gptr[r + 1] - B.gptr[r]});
     first[b + 1] = (int)mem.size();
     ord.insert(ord.end(), B.rows.begin(), B.rows.end());
@@ -673,9 +675,9 @@ static int build_team_class(shygpu_model *m) {
   }
   const bool tail = !tslot.empty();
   // teams to CTAs
-  const int G = (int)std::min<long long>(cap, ctas);
-  std::vector<int> job(m->nbasin);
-  for (int b = 0; b < m->nbasin; b++) job[b] = b;
+  G = (int)std::min<long long>(sh.capacity, ctas);
+  std::vector<int> job(NB);
+  for (int b = 0; b < NB; b++) job[b] = b;
   std::stable_sort(job.begin(), job.end(), [&](int x, int y) { return first[x + 1] - first[x] > first[y + 1] - first[y]; });
   typedef std::pair<int, int> Load;                  // teams worked so far, CTA
   std::priority_queue<Load, std::vector<Load>, std::greater<Load>> heap;
@@ -700,45 +702,69 @@ static int build_team_class(shygpu_model *m) {
     clist.insert(clist.end(), ctl[c].begin(), ctl[c].end());
     cptr[c + 1] = (int)clist.size();
   }
+  int nrow = 0;                                      // words are indexed by global row
+  for (const TeamJob &j : jobs) nrow = std::max(nrow, j.k0 + j.nk);
+  t.nrow = nrow;
+  t.nslot = (int)mem.size() + 1;                     // the last: the phantom of the timeout test
+  t.phantom = bar_test ? 1 : 0;
+  t.spin_limit = bar_test ? (1LL << 12) : zeta_team_spin_limit();
+  // every array in one allocation and one copy; the exchange words, counters
+  // and tail values start as zeros
+  std::vector<char> image;
+  auto place = [&](const void *h, size_t bytes) {
+    const size_t at = (image.size() + 255) & ~(size_t)255;
+    image.resize(at + bytes, 0);
+    if (bytes && h) memcpy(image.data() + at, h, bytes);
+    return at;
+  };
+  auto put = [&](const auto &h) { return place(h.data(), h.size() * sizeof(h[0])); };
+  const size_t o_mem = put(mem), o_cptr = put(cptr), o_clist = put(clist), o_rows = put(ord), o_dpos = put(dpos),
+               o_ghost = put(ghost), o_lcol = put(lcol), o_tptr = tail ? put(tptr) : 0, o_tcol = tail ? put(tcol) : 0,
+               o_tslot = tail ? put(tslot) : 0;
+  const size_t copied = (image.size() + 255) & ~(size_t)255;
+  const size_t n_tval = sizeof(float) * (tail ? tcol.size() : 0), n_word = sizeof(unsigned long long) * 4 * (size_t)nrow,
+               n_part = sizeof(unsigned long long) * 4 * kTeamSlotWords * (size_t)t.nslot;
+  const size_t o_part = copied, o_word = o_part + n_part, o_cnt = o_word + n_word,
+               o_tval = (o_cnt + sizeof(unsigned) * (G + 1) + 255) & ~(size_t)255, bytes = o_tval + n_tval;
+  char *base = nullptr;
+  CUDA_TRY(cudaMalloc(&base, bytes));
+  t.base = base;
+  CUDA_TRY(cudaMemcpy(base, image.data(), image.size(), cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMemset(base + copied, 0, bytes - copied));
+  t.mem = (const TeamMember *)(base + o_mem);
+  t.cptr = (const int *)(base + o_cptr);
+  t.clist = (const int *)(base + o_clist);
+  t.rows = (const int *)(base + o_rows);
+  t.dpos = (const int *)(base + o_dpos);
+  t.ghost = (const int *)(base + o_ghost);
+  t.lcol = (const unsigned short *)(base + o_lcol);
+  if (tail) {
+    t.tptr = (const int *)(base + o_tptr);
+    t.tcol = (const unsigned short *)(base + o_tcol);
+    t.tslot = (const int *)(base + o_tslot);
+    t.tval = (float *)(base + o_tval);
+  }
+  t.part = (unsigned long long *)(base + o_part);
+  t.word = (unsigned long long *)(base + o_word);
+  t.ctr = (unsigned *)(base + o_cnt);
+  t.cta_cnt = t.ctr + 1;
+  return SHY_OK;
+}
+
+// the zeta systems of every basin in one launch of the resident solver
+static int build_team_class(shygpu_model *m) {
+  std::vector<TeamJob> jobs;
+  for (int b = 0; b < m->nbasin; b++) {
+    const BasinPar &bp = m->par[b];
+    const int rows = zeta_team_share(bp.nk);
+    jobs.push_back(TeamJob{b, bp.k0, bp.nk, (bp.nk + rows - 1) / rows});
+  }
   m->zcl.emplace_back();
   ZetaClass &c = m->zcl.back();
   c.team = true;
-  c.G = G;
   c.CL = c.threads = 0;
   for (int i = 0; i < m->nbasin; i++) c.basins.push_back(i);
-  TeamPlan &t = c.tp;
-  t.nslot = (int)mem.size() + 1;                     // the last: the phantom of the timeout test
-  t.phantom = m->zbar_test ? 1 : 0;
-  t.spin_limit = m->zbar_test ? (1LL << 12) : zeta_team_spin_limit();
-  auto up = [&](auto &dst, auto &h) {
-    typename std::decay<decltype(h[0])>::type *p = nullptr;
-    const int st = upload_plan(&p, h);
-    dst = p;
-    return st;
-  };
-  ST_TRY(up(t.mem, mem));
-  ST_TRY(up(t.cptr, cptr));
-  ST_TRY(up(t.clist, clist));
-  ST_TRY(up(t.rows, ord));
-  ST_TRY(up(t.dpos, dpos));
-  ST_TRY(up(t.ghost, ghost));
-  ST_TRY(up(t.lcol, lcol));
-  if (tail) {
-    ST_TRY(up(t.tptr, tptr));
-    ST_TRY(up(t.tcol, tcol));
-    ST_TRY(up(t.tslot, tslot));
-    CUDA_TRY(cudaMalloc(&t.tval, sizeof(float) * tcol.size()));
-  }
-  const size_t nw = (size_t)4 * NKN, np = (size_t)4 * kTeamSlotWords * t.nslot;
-  CUDA_TRY(cudaMalloc(&t.word, sizeof(unsigned long long) * nw));
-  CUDA_TRY(cudaMemset(t.word, 0, sizeof(unsigned long long) * nw));
-  CUDA_TRY(cudaMalloc(&t.part, sizeof(unsigned long long) * np));
-  CUDA_TRY(cudaMemset(t.part, 0, sizeof(unsigned long long) * np));
-  CUDA_TRY(cudaMalloc(&t.ctr, sizeof(unsigned)));
-  CUDA_TRY(cudaMemset(t.ctr, 0, sizeof(unsigned)));
-  CUDA_TRY(cudaMalloc(&t.cta_cnt, sizeof(unsigned) * G));
-  CUDA_TRY(cudaMemset(t.cta_cnt, 0, sizeof(unsigned) * G));
-  return SHY_OK;
+  return make_team_plan(c.tp, c.G, zeta_team_shape(), m->rowptr_h, m->col_h, m->xy_h, jobs, m->zbar_test != 0);
 }
 
 static int build_zeta_plan_impl(shygpu_model *m, int forceCL, int forceThreads);
@@ -928,6 +954,7 @@ extern "C" int shygpu_destroy(shygpu_model *m) {
   }
   drop_graphs(m);
   free_zeta_plan(m);
+  free_team_plan(m->nh_team);
   for (int i = 0; i < kMaxZetaClasses; i++) {
     if (m->side[i]) cudaStreamDestroy(m->side[i]);
     if (m->ev_join[i]) cudaEventDestroy(m->ev_join[i]);
@@ -1079,6 +1106,23 @@ static int build_nh(shygpu_model *m, const std::vector<int> &kbas, const std::ve
   s.kbas = dkbas; s.roff = droff; s.rnode = drnode; s.rowptr = drp; s.col = dcl;
   g.rowptr = drp; g.col = dcl; g.val = s.val; g.rhs = s.rhs; g.x = s.x;
   CUDA_TRY(cudaMemset(d.qp, 0, sizeof(float) * NKN * NLV));
+  // the resident solver, where every such basin fits it
+  const TeamShape sh = csr_team_shape();
+  std::vector<float> xy((size_t)2 * nrow);
+  for (int r = 0; r < nrow; r++)
+    for (int c = 0; c < 2; c++) xy[(size_t)2 * r + c] = m->xy_h[(size_t)2 * rnode[r] + c];
+  std::vector<TeamJob> jobs;
+  for (int b = 0; b < m->nbasin; b++) {
+    const int2 rr = m->nh_rows[b];
+    if (rr.y > rr.x) jobs.push_back(TeamJob{b, rr.x, rr.y - rr.x, (rr.y - rr.x + sh.rows - 1) / sh.rows});
+  }
+  const int st = make_team_plan(m->nh_team, m->nh_TG, sh, rp, cl, xy, jobs, false);
+  if (st != SHY_OK) {
+    free_team_plan(m->nh_team);
+    m->nh_TG = 0;
+    if (st != SHY_EARG) return st;
+  }
+  m->nh_team.csr = {drp, s.val, s.rhs, s.x};
   return SHY_OK;
 }
 
@@ -1387,6 +1431,12 @@ extern "C" int shygpu_create(int32_t nbasin, const shy_basin *B, const shy_param
   if (nsc_max > 0 && (A.alloc(&d.cz_ef, (size_t)3 * NEL * nsc_max * NLV) || A.alloc(&d.cz_ef1, (size_t)3 * NEL * NLV)))
     return bail(SHY_ECAPACITY);
   if (any_up && A.upload(&d.tvdup, tvdup)) return bail(SHY_ECAPACITY);
+  m->xy_h.resize((size_t)2 * NKN);
+  for (int b = 0, k = 0; b < nbasin; b++)
+    for (int i = 0; i < B[b].nkn; i++, k++) {
+      m->xy_h[(size_t)2 * k] = B[b].xgv[i];
+      m->xy_h[(size_t)2 * k + 1] = B[b].ygv[i];
+    }
   if (m->any_nh)
     if (int st = build_nh(m, kbas, ilhkv, rowptr, col)) return bail(st);
   for (int i = 0; i < 2; i++) {
@@ -1398,12 +1448,6 @@ extern "C" int shygpu_create(int32_t nbasin, const shy_basin *B, const shy_param
   if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess)
     return bail(fail(SHY_ECUDA, "stream creation failed"));
   // zeta solver launch shape: one cluster per basin, about 2k rows per CTA
-  m->xy_h.resize((size_t)2 * NKN);
-  for (int b = 0, k = 0; b < nbasin; b++)
-    for (int i = 0; i < B[b].nkn; i++, k++) {
-      m->xy_h[(size_t)2 * k] = B[b].xgv[i];
-      m->xy_h[(size_t)2 * k + 1] = B[b].ygv[i];
-    }
   m->rowptr_h = rowptr;
   m->col_h = col;
   if (cudaEventCreateWithFlags(&m->ev_fork, cudaEventDisableTiming) != cudaSuccess)
@@ -1647,6 +1691,15 @@ static int enqueue_nh(shygpu_model *m, const Dev &d) {
   const NhSys &s = m->nh;
   launch_nh(d, s, 0, m->stream);
   launch_nh(d, s, 1, m->stream);
+  if (m->nh_TG > 0) {                // the resident solver, from a zero guess
+    ZetaArgs za{};
+    za.inner_rtol = m->inner_rtol; za.tol_frac = 0.25f; za.max_outer = m->max_outer;
+    cudaError_t e = launch_csr_team(d, za, m->nh_team, m->nh_TG, m->stream);
+    if (e != cudaSuccess) return fail(SHY_ECUDA, "non-hydrostatic solve launch: %s", cudaGetErrorString(e));
+    launch_nh(d, s, 2, m->stream);
+    launch_nh(d, s, 3, m->stream);
+    return SHY_OK;
+  }
   CUDA_TRY(cudaMemsetAsync(s.x, 0, sizeof(float) * s.nrow, m->stream));
   for (int b = 0; b < m->nbasin; b++) {
     const int2 rr = m->nh_rows[b];
@@ -1670,6 +1723,7 @@ static int enqueue_nh(shygpu_model *m, const Dev &d) {
 static int nh_launches(const shygpu_model *m) {
   if (!m->any_nh) return 0;
   int n = 4;
+  if (m->nh_TG > 0) return n + 1;
   for (const int2 &r : m->nh_rows) n += r.y > r.x ? 1 : 0;
   return n;
 }

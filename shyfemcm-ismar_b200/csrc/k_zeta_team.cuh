@@ -239,16 +239,19 @@ __device__ __forceinline__ float at4(const float *a, unsigned pair, int k) {
 }
 
 // buffer of exchange number xi >= 1 (0 uses buffers 0, 2 and 3)
-__device__ __forceinline__ u64 *team_buf(const TeamPlan &tp, const Dev &d, unsigned xi) {
-  return tp.word + (size_t)(xi & 1u) * d.NKN;
+__device__ __forceinline__ u64 *team_buf(const TeamPlan &tp, unsigned xi) {
+  return tp.word + (size_t)(xi & 1u) * tp.nrow;
 }
 
 // SYM: CG on the symmetrically scaled system S A S; else BiCGStab (van der
 // Vorst 1992) on A D^-1 (right Jacobi preconditioning), for systems with
 // Coriolis or dry elements, and the repeat loop of wetting and drying
 // (hydrodynamic.f90:374-404).  Both scaled matrices have a unit diagonal.
-template <int NT, int R, int GR, bool SYM>
+// K: off-diagonal entries in a row's block.  CSR: not the zeta system but one
+// given in CSR form (TeamPlan::csr), from a zero guess: the 3D pressure.
+template <int NT, int R, int GR, int K, bool SYM, bool CSR>
 __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPlan tp) {
+  static_assert(!(SYM && CSR), "the 3D system is not symmetric");
   typedef TeamShared<NT, R, GR> SH;
   __shared__ SH sh;
   const int tid = threadIdx.x;
@@ -258,7 +261,7 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
   const unsigned launch = tp.cta_cnt[blockIdx.x] + 1u, abortv = launch;
   bool dead = false;
   if (tid == 0) sh.ok = 1;
-  if (blockIdx.x == 0 && tid == 0 && d.imax) { *d.imax = 0; *d.subj = 0; }
+  if (!CSR && blockIdx.x == 0 && tid == 0 && d.imax) { *d.imax = 0; *d.subj = 0; }
 
   for (int q = q0; q < q1; q++) {
     const int me = tp.clist[q];
@@ -272,11 +275,11 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
     const int n = M.nrow, nr = (n + NT - 1) / NT;   // rows, rows a thread at most
     const int echunk = (P.ne + M.T - 1) / M.T;   // this member's elements (wetting and drying)
     const int ea = P.e0 + min(P.ne, M.rank * echunk), eb = min(P.e0 + P.ne, ea + echunk);
-    if (M.rank == 0 && tid < kMaxScal) O.stab[tid] = 0.f;   // reset for k_stab's max
+    if (!CSR && M.rank == 0 && tid < kMaxScal) O.stab[tid] = 0.f;   // reset for k_stab's max
     const float dtf = (float)P.dt;
     // wetting and drying: a domain that can change with the solution
-    const bool wd = !SYM && wd_basin(P) && !za.explicit_mode;
-    const bool extrap = za.zprev != nullptr && O.steps > 0 && !wd;
+    const bool wd = !SYM && !CSR && wd_basin(P) && !za.explicit_mode;
+    const bool extrap = !CSR && za.zprev != nullptr && O.steps > 0 && !wd;
     // a barrier of the team that also makes its global writes visible; sums
     // one value
     auto team_barrier = [&](double &v) -> bool {
@@ -308,6 +311,9 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
     }
     // the guess: the old level, in repeats the last solution
     const float *guess = rep == 0 ? za.zguess : d.zn;
+    const int *rowptr = CSR ? tp.csr.rowptr : d.rowptr;
+    double *val64 = CSR ? const_cast<double *>(tp.csr.val) : d.val64;
+    const double *rhs64 = CSR ? tp.csr.rhs : d.rhs64;
     auto level = [&](int i) { return (double)(wd ? __ldcg(guess + i) : guess[i]); };
 
     // ---- assembly (FP64 sums in element order), Jacobi scale, and the
@@ -329,57 +335,64 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
       if (j >= n) continue;
       ri[r] = tp.rows[M.row0 + j];
       const int i = ri[r] & 0x7fffffff;
-      const int s0 = d.rowptr[i];
-      const int dn = tp.dpos[M.row0 + j], dp = dn & 0xff, nd = dn >> 8;   // diagonal's place, off-diagonal entries
-      double diag = 0., rhs = 0.;
-      const int p1 = d.inc_ptr[i + 1];
-      for (int p0 = d.inc_ptr[i]; p0 < p1; p0 += 8) {   // eight elements at a time, their loads in flight together
-        float ha[8], hb[8];
+      double diag = 0., tA, tB = 0.;
+      if constexpr (CSR) {
+        diag = val64[rowptr[i] + (tp.dpos[M.row0 + j] & 0xff)];
+        tA = rhs64[i];                           // the guess is zero
+      } else {
+        const int s0 = d.rowptr[i];
+        const int dn = tp.dpos[M.row0 + j], dp = dn & 0xff, nd = dn >> 8;   // diagonal's place, off-diagonal entries
+        double rhs = 0.;
+        const int p1 = d.inc_ptr[i + 1];
+        for (int p0 = d.inc_ptr[i]; p0 < p1; p0 += 8) {   // eight elements at a time, their loads in flight together
+          float ha[8], hb[8];
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-          const bool in = p0 + k < p1;
-          const int e3 = in ? d.inc[p0 + k] : 0, e = e3 / 3, ii = e3 - 3 * e;
-          ha[k] = in ? elem(za.hia, 4 * ii, e) : 0.f;
-          hb[k] = in ? elem(za.hik, ii, e) : 0.f;
+          for (int k = 0; k < 8; k++) {
+            const bool in = p0 + k < p1;
+            const int e3 = in ? d.inc[p0 + k] : 0, e = e3 / 3, ii = e3 - 3 * e;
+            ha[k] = in ? elem(za.hia, 4 * ii, e) : 0.f;
+            hb[k] = in ? elem(za.hik, ii, e) : 0.f;
+          }
+#pragma unroll
+          for (int k = 0; k < 8; k++) { diag += (double)ha[k]; rhs += (double)hb[k]; }
         }
-#pragma unroll
-        for (int k = 0; k < 8; k++) { diag += (double)ha[k]; rhs += (double)hb[k]; }
-      }
-      // adjust_mass_flux (bnd_routines.f90:1185-1210): no flux enters a node
-      // out of the system
-      if (!(wd && d.inod[i] == -2)) rhs += (double)(dtf * d.rqv[i]);
-      d.rhs64[i] = rhs;
-      const double zg = level(i);
-      if (za.explicit_mode) {
-        const double x0 = diag != 0. ? rhs / diag : 0.;
-        d.x64[i] = x0;
-        d.zn[i] = (float)x0;
-        continue;
-      }
-      d.val64[s0 + dp] = diag;
-      double tA = rhs - diag * zg, tB = extrap ? rhs - diag * (2. * zg - (double)za.zprev[i]) : 0.;
-      // an off-diagonal entry: the elements on both sides of its edge (any
-      // more in order after them)
-      auto entry = [&](int k) {
-        const int sl = s0 + k + (k >= dp);
-        const int q0s = d.slot_ptr[sl], q1s = d.slot_ptr[sl + 1];
-        const int srcA = d.slot_src[q0s], srcB = q1s - q0s > 1 ? d.slot_src[q0s + 1] : -1;
-        const int eA = srcA / 9, eB = srcB < 0 ? 0 : srcB / 9;
-        double a = (double)elem(za.hia, srcA - 9 * eA, eA);
-        if (srcB >= 0) a += (double)elem(za.hia, srcB - 9 * eB, eB);
-        for (int t = q0s + 2; t < q1s; t++) {
-          const int e = d.slot_src[t] / 9;
-          a += (double)elem(za.hia, d.slot_src[t] - 9 * e, e);
+        // adjust_mass_flux (bnd_routines.f90:1185-1210): no flux enters a node
+        // out of the system
+        if (!(wd && d.inod[i] == -2)) rhs += (double)(dtf * d.rqv[i]);
+        d.rhs64[i] = rhs;
+        const double zg = level(i);
+        if (za.explicit_mode) {
+          const double x0 = diag != 0. ? rhs / diag : 0.;
+          d.x64[i] = x0;
+          d.zn[i] = (float)x0;
+          continue;
         }
-        const int c = d.col[sl];
-        d.val64[sl] = a;
-        tA -= a * level(c);
-        if (extrap) tB -= a * (2. * level(c) - (double)za.zprev[c]);
-      };
+        d.val64[s0 + dp] = diag;
+        tA = rhs - diag * zg;
+        tB = extrap ? rhs - diag * (2. * zg - (double)za.zprev[i]) : 0.;
+        // an off-diagonal entry: the elements on both sides of its edge (any
+        // more in order after them)
+        auto entry = [&](int k) {
+          const int sl = s0 + k + (k >= dp);
+          const int q0s = d.slot_ptr[sl], q1s = d.slot_ptr[sl + 1];
+          const int srcA = d.slot_src[q0s], srcB = q1s - q0s > 1 ? d.slot_src[q0s + 1] : -1;
+          const int eA = srcA / 9, eB = srcB < 0 ? 0 : srcB / 9;
+          double a = (double)elem(za.hia, srcA - 9 * eA, eA);
+          if (srcB >= 0) a += (double)elem(za.hia, srcB - 9 * eB, eB);
+          for (int t = q0s + 2; t < q1s; t++) {
+            const int e = d.slot_src[t] / 9;
+            a += (double)elem(za.hia, d.slot_src[t] - 9 * e, e);
+          }
+          const int c = d.col[sl];
+          d.val64[sl] = a;
+          tA -= a * level(c);
+          if (extrap) tB -= a * (2. * level(c) - (double)za.zprev[c]);
+        };
 #pragma unroll
-      for (int k = 0; k < 8; k++)
-        if (k < nd) entry(k);
-      for (int k = 8; k < nd; k++) entry(k);
+        for (int k = 0; k < 8; k++)
+          if (k < nd) entry(k);
+        for (int k = 8; k < nd; k++) entry(k);
+      }
       const float sd = SYM ? (diag > 0. ? (float)(1. / sqrt(diag)) : 1.f) : (diag != 0. ? (float)(1. / diag) : 1.f);
       sh.sd[j] = sd;
       rsA[r] = (float)(SYM ? (double)sd * tA : tA);
@@ -398,10 +411,10 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
     for (int r = 0; r < R; r++)
       if (ri[r] < 0) {
         const size_t i = (size_t)(ri[r] & 0x7fffffff);
-        word_put(team_buf(tp, d, xi) + i, __float_as_uint(sh.sd[r * NT + tid]), ep);
-        if (rep == 0) word_put(team_buf(tp, d, xi + 1u) + i, 0u, ep);   // every launch renews every word
-        word_put(tp.word + 2 * (size_t)d.NKN + i, __float_as_uint(rsA[r]), ep);
-        word_put(tp.word + 3 * (size_t)d.NKN + i, __float_as_uint(rsB[r]), ep);
+        word_put(team_buf(tp, xi) + i, __float_as_uint(sh.sd[r * NT + tid]), ep);
+        if (rep == 0) word_put(team_buf(tp, xi + 1u) + i, 0u, ep);   // every launch renews every word
+        word_put(tp.word + 2 * (size_t)tp.nrow + i, __float_as_uint(rsA[r]), ep);
+        word_put(tp.word + 3 * (size_t)tp.nrow + i, __float_as_uint(rsB[r]), ep);
       }
     {
       const double y0 = warp_sum2(v4[0], v4[1]), y1 = warp_sum2(v4[2], v4[3]);
@@ -423,7 +436,7 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
       if (jg < M.nghost) {
         gi[g] = tp.ghost[M.ghost0 + jg];
         const u64 *p = tp.word + gi[g];
-        const u64 *const pw[3] = {team_buf(tp, d, xi) + gi[g], p + 2 * (size_t)d.NKN, p + 3 * (size_t)d.NKN};
+        const u64 *const pw[3] = {team_buf(tp, xi) + gi[g], p + 2 * (size_t)tp.nrow, p + 3 * (size_t)tp.nrow};
         unsigned h[3];
         ok = words_wait(tp, pw, ep, abortv, h) && ok;
         sd = __uint_as_float(h[0]);
@@ -460,37 +473,43 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
       for (int r = 0; r < R; r++) {
         const int j = r * NT + tid;
         rr[r] = useB ? rsB[r] : rsA[r];
-        if (j < n) sh.x[j] = start(ri[r] & 0x7fffffff);
+        if (j < n) sh.x[j] = CSR ? 0. : start(ri[r] & 0x7fffffff);
       }
 #pragma unroll
       for (int g = 0; g < GR; g++) {
         if (useB) gr[g] = grB[g];
-        if (gi[g] >= 0) sh.x[NT * R + g * NT + gtid] = start(gi[g]);
+        if (gi[g] >= 0) sh.x[NT * R + g * NT + gtid] = CSR ? 0. : start(gi[g]);
       }
     }
-    float val[R][8];
-    unsigned col[R][4];
+    float val[R][K];
+    unsigned col[R][K / 2];
 #pragma unroll
     for (int r = 0; r < R; r++) {
       const int j = r * NT + tid;
 #pragma unroll
-      for (int k = 0; k < 8; k++) val[r][k] = 0.f;
+      for (int k = 0; k < K; k++) val[r][k] = 0.f;
 #pragma unroll
-      for (int k = 0; k < 4; k++) col[r][k] = 0u;
+      for (int k = 0; k < K / 2; k++) col[r][k] = 0u;
       if (j >= n) continue;
-      const uint4 c4 = __ldg(reinterpret_cast<const uint4 *>(tp.lcol) + M.row0 + j);
-      col[r][0] = c4.x; col[r][1] = c4.y; col[r][2] = c4.z; col[r][3] = c4.w;
+      if constexpr (K == 8) {
+        const uint4 c4 = __ldg(reinterpret_cast<const uint4 *>(tp.lcol) + M.row0 + j);
+        col[r][0] = c4.x; col[r][1] = c4.y; col[r][2] = c4.z; col[r][3] = c4.w;
+      } else {
+#pragma unroll
+        for (int k = 0; k < K / 2; k++)
+          col[r][k] = __ldg(reinterpret_cast<const unsigned *>(tp.lcol) + (size_t)(M.row0 + j) * (K / 2) + k);
+      }
       const int i = ri[r] & 0x7fffffff;
       const int dn = tp.dpos[M.row0 + j], dp = dn & 0xff, nd = dn >> 8;
       const double sdi = SYM ? (double)sh.sd[j] : 1.;
-      const double *a = d.val64 + d.rowptr[i];
+      const double *a = val64 + rowptr[i];
 #pragma unroll
-      for (int k = 0; k < 8; k++)
+      for (int k = 0; k < K; k++)
         if (k < nd)
           val[r][k] = (float)(a[k + (k >= dp)] * sdi * (double)at4(sh.sd, col[r][k >> 1], k));
       if (tp.tptr)                               // a long row's tail
         for (int t = tp.tptr[M.row0 + j]; t < tp.tptr[M.row0 + j + 1]; t++)
-          tp.tval[t] = (float)(d.val64[tp.tslot[t]] * sdi * (double)sh.sd[tp.tcol[t]]);
+          tp.tval[t] = (float)(val64[tp.tslot[t]] * sdi * (double)sh.sd[tp.tcol[t]]);
     }
 
     // the scaled matrix times u for the own rows: the unit diagonal times
@@ -501,7 +520,7 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
         w[r] = x[r];
         if (r >= nr) continue;
 #pragma unroll
-        for (int k = 0; k < 8; k++)
+        for (int k = 0; k < K; k++)
           w[r] += val[r][k] * at4(sh.u, col[r][k >> 1], k);
         if (tp.tptr && r * NT + tid < n)
           for (int t = tp.tptr[M.row0 + r * NT + tid]; t < tp.tptr[M.row0 + r * NT + tid + 1]; t++)
@@ -514,7 +533,7 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
     auto exchange = [&](const float (&w)[R], float (&gw)[GR], const auto &v, auto post) -> bool {
       constexpr int NP = sizeof(v) / (2 * sizeof(double));
       ep = number();
-      u64 *buf = team_buf(tp, d, xi);
+      u64 *buf = team_buf(tp, xi);
 #pragma unroll
       for (int r = 0; r < R; r++)
         if (ri[r] < 0) word_put(buf + (ri[r] & 0x7fffffff), __float_as_uint(w[r]), ep);
@@ -541,7 +560,7 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
     };
 
     for (outer = 0;;) {
-      if (sh.rn <= sh.tol || outer >= za.max_outer) break;
+      if (sh.rn <= sh.tol || outer >= za.max_outer || (CSR && iters >= P.maxit)) break;
       if (tid == 0) {
         // the FP32 sweep's target, moved into the norm of the residual it works on
         const double it0 = fmax((double)za.inner_rtol * sh.rn, tfrac(za) * sh.tol);
@@ -677,7 +696,7 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
                 sh.fo = (float)om;
                 sh.fb = (float)((rho / sh.rho) * (sh.alpha / om));
                 sh.stop = !(r2 > sh.itol2) || !(r2 == r2) || om == 0. || sh.alpha == 0. || rho == 0. ||
-                          inner >= P.maxit;
+                          (CSR ? iters + 1 : inner) >= P.maxit;
                 sh.rho = rho;
               })) { dead = true; break; }
           const float fw = sh.fo;
@@ -716,14 +735,14 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
         if (j >= n) continue;
         const int i = ri[r] & 0x7fffffff;
         const int dn = tp.dpos[M.row0 + j], dp = dn & 0xff, nd = dn >> 8;
-        const double *a = d.val64 + d.rowptr[i];
-        double t = d.rhs64[i] - a[dp] * sh.x[j];
+        const double *a = val64 + rowptr[i];
+        double t = rhs64[i] - a[dp] * sh.x[j];
 #pragma unroll
-        for (int k = 0; k < 8; k++)
+        for (int k = 0; k < K; k++)
           if (k < nd) t -= a[k + (k >= dp)] * sh.x[(k & 1 ? col[r][k >> 1] >> 16 : col[r][k >> 1] & 0xffffu) >> 2];
         if (tp.tptr)
           for (int q2 = tp.tptr[M.row0 + j]; q2 < tp.tptr[M.row0 + j + 1]; q2++)
-            t -= d.val64[tp.tslot[q2]] * sh.x[tp.tcol[q2]];
+            t -= val64[tp.tslot[q2]] * sh.x[tp.tcol[q2]];
         rr[r] = (float)(SYM ? (double)sh.sd[j] * t : t);
         v[0] += t * t;
         v[1] += (double)rr[r] * rr[r];
@@ -738,7 +757,10 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
     refine += outer;
 #pragma unroll
     for (int r = 0; r < R; r++)
-      if (r * NT + tid < n) d.zn[ri[r] & 0x7fffffff] = (float)sh.x[r * NT + tid];
+      if (r * NT + tid < n) {
+        if constexpr (CSR) tp.csr.x[ri[r] & 0x7fffffff] = (float)sh.x[r * NT + tid];
+        else d.zn[ri[r] & 0x7fffffff] = (float)sh.x[r * NT + tid];
+      }
     if (!wd) break;
     // setweg(1): elements with a vertex below hzmin leave; then the step
     // counters, every element on the first pass of the step (a new time)
@@ -755,10 +777,17 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
     if (dead) break;
     if (za.explicit_mode) continue;
     if (tid == 0 && M.rank == 0) {
-      O.iters = iters;
-      O.refinements = refine;
-      O.resid0 = sh.resid0;
-      O.resid = sh.rn;
+      if constexpr (CSR) {
+        O.nh_iters = iters;
+        O.nh_refinements = refine;
+        O.nh_resid0 = sh.resid0;
+        O.nh_resid = sh.rn;
+      } else {
+        O.iters = iters;
+        O.refinements = refine;
+        O.resid0 = sh.resid0;
+        O.resid = sh.rn;
+      }
       if (!(sh.rn <= sh.tol)) set_status(&O, SHY_ENOCONV);
     }
     __syncthreads();                             // sh is reused by the next basin

@@ -132,6 +132,9 @@ struct TeamMember {
 // of one word per row; part: two buffers of a
 // slot per member and the phantom, for its own sums and for the totals.
 struct TeamPlan {
+  // the system of the CSR instance: FP64 matrix and right-hand side, solution
+  struct { const int *rowptr; const double *val, *rhs; float *x; } csr = {nullptr, nullptr, nullptr, nullptr};
+  void *base = nullptr;            // the allocation that holds the arrays below
   const TeamMember *mem = nullptr;
   const int *cptr = nullptr, *clist = nullptr;
   const int *rows = nullptr, *dpos = nullptr, *ghost = nullptr;
@@ -140,6 +143,7 @@ struct TeamPlan {
   float *tval = nullptr;
   unsigned long long *word = nullptr, *part = nullptr;
   unsigned *ctr = nullptr, *cta_cnt = nullptr;   // abort word; launches made, per CTA
+  int nrow = 0;                    // rows of the whole system
   int nslot = 0;                   // the last one the phantom's
   int phantom = 0;                 // 1: every exchange waits for a member that does not exist (timeout test)
   long long spin_limit = 0;        // polls before a wait gives up
@@ -167,10 +171,18 @@ cudaError_t launch_zeta_grid(const Dev &d, const ZetaArgs &za, const GridPlan &g
                              size_t smem, cudaStream_t st);
 // the resident variant: G CTAs, cooperative
 cudaError_t launch_zeta_team(const Dev &d, const ZetaArgs &za, const TeamPlan &tp, int G, cudaStream_t st);
-int zeta_team_capacity();    // its CTAs that fit the device at once (0 on error)
-int zeta_team_rows();        // rows a CTA holds at most
+// its CSR instance: the systems of the 3D pressure
+cudaError_t launch_csr_team(const Dev &d, const ZetaArgs &za, const TeamPlan &tp, int G, cudaStream_t st);
+// what a CTA of the resident solver holds
+struct TeamShape {
+  int rows;      // rows at most (the first place of a ghost)
+  int ghosts;    // ghost copies at most
+  int entries;   // off-diagonal entries in a row's block
+  int capacity;  // CTAs that fit the device at once (0 on error)
+};
+TeamShape zeta_team_shape();
+TeamShape csr_team_shape();
 int zeta_team_share(int nk); // rows a CTA gets at most in a basin of nk rows
-int zeta_team_ghosts();      // ghost rows a CTA holds
 long long zeta_team_spin_limit();
 // CTAs of k_zeta_grid that fit the device at once (0 on error)
 int zeta_grid_capacity(bool staged, size_t smem);

@@ -60,10 +60,17 @@ cudaError_t launch_zeta_grid(const Dev &d, const ZetaArgs &za, const GridPlan &g
              : cudaLaunchKernelEx(&cfg, k_zeta_grid<512, false, false>, d, za, gp);
 }
 
-constexpr int kTeamNT = 512, kTeamR = 4, kTeamGR = 1;
+constexpr int kTeamNT = 512;
 constexpr long long kTeamSpinLimit = 1LL << 22;   // polls of a word: seconds
+// the zeta system (rows of up to eight neighbours in the block), and the 3D
+// system (three layers of them and the two of the own column, less the row
+// itself, for up to eight neighbours)
+constexpr auto kZetaSym = k_zeta_team<kTeamNT, 4, 1, 8, true, false>;
+constexpr auto kZetaGen = k_zeta_team<kTeamNT, 4, 1, 8, false, false>;
+constexpr auto kCsrGen = k_zeta_team<kTeamNT, 1, 2, 26, false, true>;
 
-cudaError_t launch_zeta_team(const Dev &d, const ZetaArgs &za, const TeamPlan &tp, int G, cudaStream_t st) {
+static cudaError_t launch_team(void (*kernel)(Dev, ZetaArgs, TeamPlan), const Dev &d, const ZetaArgs &za,
+                               const TeamPlan &tp, int G, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   cfg.gridDim = dim3(G, 1, 1);
@@ -73,30 +80,35 @@ cudaError_t launch_zeta_team(const Dev &d, const ZetaArgs &za, const TeamPlan &t
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return za.sym ? cudaLaunchKernelEx(&cfg, k_zeta_team<kTeamNT, kTeamR, kTeamGR, true>, d, za, tp)
-                : cudaLaunchKernelEx(&cfg, k_zeta_team<kTeamNT, kTeamR, kTeamGR, false>, d, za, tp);
+  return cudaLaunchKernelEx(&cfg, kernel, d, za, tp);
 }
 
-int zeta_team_capacity() {
-  int dev = 0, nsm = 0, na = 0, nb = 0;
+cudaError_t launch_zeta_team(const Dev &d, const ZetaArgs &za, const TeamPlan &tp, int G, cudaStream_t st) {
+  return launch_team(za.sym ? kZetaSym : kZetaGen, d, za, tp, G, st);
+}
+
+cudaError_t launch_csr_team(const Dev &d, const ZetaArgs &za, const TeamPlan &tp, int G, cudaStream_t st) {
+  return launch_team(kCsrGen, d, za, tp, G, st);
+}
+
+static int team_capacity(void (*kernel)(Dev, ZetaArgs, TeamPlan)) {
+  int dev = 0, nsm = 0, nb = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&na, k_zeta_team<kTeamNT, kTeamR, kTeamGR, true>, kTeamNT, 0) !=
-          cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_zeta_team<kTeamNT, kTeamR, kTeamGR, false>, kTeamNT, 0) !=
-          cudaSuccess)
-    return 0;
-  return std::min(std::min(na, nb) * nsm, kTeamNT);      // one thread polls each member of a team
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, kTeamNT, 0) != cudaSuccess) return 0;
+  return std::min(nb * nsm, kTeamNT);      // one thread polls each member of a team
 }
-int zeta_team_rows() { return kTeamNT * kTeamR; }
+TeamShape zeta_team_shape() {
+  return TeamShape{kTeamNT * 4, kTeamNT, 8, std::min(team_capacity(kZetaSym), team_capacity(kZetaGen))};
+}
+TeamShape csr_team_shape() { return TeamShape{kTeamNT, 2 * kTeamNT, 26, team_capacity(kCsrGen)}; }
 // Rows a CTA gets: 1024 in basins of up to 40 shares, where a team's
 // latency matters (7k rows: 0.31 ms a solve on 7 CTAs, 0.38 ms on 4), 2048
 // in larger ones, where more members only make the exchange slower (250k
 // rows: 0.42 ms on 123, 0.66 ms on 245) and the ensemble's basins take turns
 // on the CTAs (64 basins: 2.8 ms against 3.2 ms).  It depends on the basin
 // alone, so that its bits do.
-int zeta_team_share(int nk) { return nk <= 40960 ? kTeamNT * kTeamR / 2 : kTeamNT * kTeamR; }
-int zeta_team_ghosts() { return kTeamNT * kTeamGR; }
+int zeta_team_share(int nk) { return nk <= 40960 ? kTeamNT * 2 : kTeamNT * 4; }
 long long zeta_team_spin_limit() { return kTeamSpinLimit; }
 
 size_t zeta_grid_stage_smem(bool c16) { return 128 + 2 * (size_t)stage_layout(c16 ? 16 : 32).bytes; }
