@@ -1,5 +1,5 @@
 // k_column_t.cuh -- the column kernel with one thread per element column,
-// for shallow columns (at most L layers): hydro_transports / hydro_intern /
+// for columns of at most L layers: hydro_transports / hydro_intern /
 // hydro_zeta element part (hydrodynamic.f90:758-864, 868-1416, 488-733).
 //
 // The same arithmetic as k_column (k_column.cuh), which spreads a column's
@@ -32,10 +32,22 @@ namespace shy {
 // pressure); without them the plain barotropic column keeps fewer registers
 // and runs six CTAs per SM (measured faster than five, where it has no
 // spills, on the 10-layer ensemble).
+// L > 16 (staged only): the sweep's coefficients stay in shared memory as
+// well and the layer loop is not unrolled (four arrays of 32 layers would
+// not fit the registers); dp2 takes the place of the thickness already
+// read.  One warp per CTA, six arrays of 32 columns at an odd stride (no bank
+// conflicts), eight warps per SM.  Against the warp segment per column
+// (k_column), whose 32 lanes repeat the element's FP64 terms and reduce the
+// system in five rounds of shuffles: 0.48 against 1.17 ms on 500k columns of 30 layers,
+// 74 against 115 us on 39k columns of 20 (42% of the layers wet).  Shorter columns
+// stay in registers (10 layers, 4.2M columns: 0.70 ms, 1.05 ms this way).
 template <int L, bool COR, bool ADV, bool W = false, bool XT = true>
-__global__ void __launch_bounds__(128, W ? (XT ? 4 : 6) : 3) k_column_t(Dev d) {
+__global__ void __launch_bounds__(L > 16 ? 32 : 128, L > 16 ? 8 : (W ? (XT ? 4 : 6) : 3)) k_column_t(Dev d) {
+  constexpr bool BIG = L > 16;
   static_assert(!(W && COR), "the staged form has no Coriolis instance");
-  __shared__ float sbuf[W ? 4 : 1][W ? 3 : 1][W ? 32 * L : 1];
+  static_assert(W || !BIG, "long columns are staged");
+  __shared__ float sbuf[W && !BIG ? 4 : 1][W && !BIG ? 3 : 1][W && !BIG ? 32 * L : 1];
+  extern __shared__ float col_dyn[];                  // BIG: six arrays of 32 columns
   const int e0 = blockIdx.x * blockDim.x + threadIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if constexpr (!W) {
@@ -48,9 +60,23 @@ __global__ void __launch_bounds__(128, W ? (XT ? 4 : 6) : 3) k_column_t(Dev d) {
   const bool valid = !W || lane < nw;
   const int e = valid ? e0 : w0;                      // spare lanes work a copy of the first column
   const int NLV = d.NLV;
-  float *bH = sbuf[warp][0], *bU = sbuf[warp][1], *bV = sbuf[warp][2];
-  const int ol = lane * NLV;                          // this thread's column in the buffers
-  if constexpr (W) {
+  const int LS = BIG ? NLV | 1 : NLV;                 // stride of the columns in the buffers
+  const int sw = BIG ? 0 : warp;
+  float *bH = BIG ? col_dyn : sbuf[sw][0], *bU = BIG ? bH + 32 * LS : sbuf[sw][W && !BIG ? 1 : 0],
+        *bV = BIG ? bU + 32 * LS : sbuf[sw][W && !BIG ? 2 : 0];
+  float *bC = bV + 32 * LS, *bP = bC + 32 * LS, *bQ = bP + 32 * LS;   // BIG: cp, dp0, dp1
+  const int ol = lane * LS;                           // this thread's column in the buffers
+  if constexpr (BIG) {
+    const size_t base = (size_t)w0 * NLV;
+#pragma unroll 4
+    for (int c = 0; c < 32; c++) {                    // spare lanes' columns read as zero
+      const bool in = c < nw && lane < NLV;
+      const size_t q = base + (size_t)c * NLV + lane;
+      const float a = in ? d.heo[q] : 0.f, b = in ? d.uo[q] : 0.f, v = in ? d.vo[q] : 0.f;
+      if (lane < NLV) { bH[c * LS + lane] = a; bU[c * LS + lane] = b; bV[c * LS + lane] = v; }
+    }
+    __syncwarp();
+  } else if constexpr (W) {
     const size_t base = (size_t)w0 * NLV;
     const int cnt = nw * NLV;
     for (int j = lane; j < 32 * NLV; j += 32) {      // spare lanes' columns read as zero
@@ -113,8 +139,11 @@ __global__ void __launch_bounds__(128, W ? (XT ? 4 : 6) : 3) k_column_t(Dev d) {
   const float raux = P.grav / P.rowass;
 
   // forward Thomas sweep as the layer coefficients are formed
-  float cp[L];
-  float dp0[L], dp1[L], dp2[L];            // real: rhs ppx, ppy, h
+  constexpr int LR = BIG ? 1 : L;          // BIG: kept in shared memory
+  float cp[LR];
+  float dp0[LR], dp1[LR], dp2[LR];         // real: rhs ppx, ppy, h
+#define SWEEP(r, m, i) (BIG ? m[ol + (i)] : r[BIG ? 0 : (i)])
+  float hprev = 0.f;                       // the thickness of the layer above
   float2 cpc[COR ? L : 1], dq0[COR ? L : 1], dq1[COR ? L : 1];   // complex: ppx+i ppy, h
   float adv_wtop = 0.f;                    // vertical momentum advection: w at the layer's top
   float alev_t = P.vismol;
@@ -128,15 +157,14 @@ __global__ void __launch_bounds__(128, W ? (XT ? 4 : 6) : 3) k_column_t(Dev d) {
 #pragma unroll
     for (int ii = 0; ii < 3; ii++) hoi[ii] = -(double)d.zo[kn[ii]];
   float pxs = 0.f, pys = 0.f;              // their running sums from the surface
-#pragma unroll
-  for (int l = 0; l < L; l++) {
-    if (l >= ilevel) break;
+  auto down = [&](const int l) __attribute__((always_inline)) {
     const bool bfirst = l == 0, blast = l == ilevel - 1;
     const float hhi = COL_H(l), uui = COL_U(l), vvi = COL_V(l);
     float hhip = blast ? 0.f : COL_H(l + 1 < L ? l + 1 : l);
     float uuip = blast ? uui : COL_U(l + 1 < L ? l + 1 : l);
     float vvip = blast ? vvi : COL_V(l + 1 < L ? l + 1 : l);
-    const float hhim = bfirst ? 0.f : COL_H(l > 0 ? l - 1 : 0);
+    const float hhim = BIG ? hprev : (bfirst ? 0.f : COL_H(l > 0 ? l - 1 : 0));
+    hprev = hhi;
     const float uuim = bfirst ? uui : COL_U(l > 0 ? l - 1 : 0);
     const float vvim = bfirst ? vvi : COL_V(l > 0 ? l - 1 : 0);
     const float rhact = hhi > 0.f ? 1.f / hhi : 0.f;
@@ -280,12 +308,17 @@ __global__ void __launch_bounds__(128, W ? (XT ? 4 : 6) : 3) k_column_t(Dev d) {
     const float up = blast ? 0.f : -bb;
     const float dg = 1.f + aa;
     if constexpr (!COR) {
-      const float cprev = bfirst ? 0.f : cp[l > 0 ? l - 1 : 0];
+      const int m = l > 0 ? l - 1 : 0;
+      const float cprev = bfirst ? 0.f : SWEEP(cp, bC, m);
       const float rden = 1.f / (dg - lo * cprev);
-      cp[l] = up * rden;
-      dp0[l] = (ppx - (bfirst ? 0.f : lo * dp0[l > 0 ? l - 1 : 0])) * rden;
-      dp1[l] = (ppy - (bfirst ? 0.f : lo * dp1[l > 0 ? l - 1 : 0])) * rden;
-      dp2[l] = (hhi - (bfirst ? 0.f : lo * dp2[l > 0 ? l - 1 : 0])) * rden;
+      const float q0 = (ppx - (bfirst ? 0.f : lo * SWEEP(dp0, bP, m))) * rden;
+      const float q1 = (ppy - (bfirst ? 0.f : lo * SWEEP(dp1, bQ, m))) * rden;
+      const float q2 = (hhi - (bfirst ? 0.f : lo * SWEEP(dp2, bH, m))) * rden;
+      if constexpr (BIG) {
+        bC[ol + l] = up * rden; bP[ol + l] = q0; bQ[ol + l] = q1; bH[ol + l] = q2;
+      } else {
+        cp[l] = up * rden; dp0[l] = q0; dp1[l] = q1; dp2[l] = q2;
+      }
     } else {
       const float2 cprev = bfirst ? make_float2(0.f, 0.f) : cpc[l > 0 ? l - 1 : 0];
       const float2 den = make_float2(dg - lo * cprev.x, (float)gamma - lo * cprev.y);
@@ -301,23 +334,32 @@ __global__ void __launch_bounds__(128, W ? (XT ? 4 : 6) : 3) k_column_t(Dev d) {
       dq0[l] = cmulf(r0, rden);
       dq1[l] = cmulf(r1, rden);
     }
+  };
+  if constexpr (BIG) {
+#pragma unroll 1
+    for (int l = 0; l < ilevel; l++) down(l);
+  } else {
+#pragma unroll
+    for (int l = 0; l < L; l++) {
+      if (l >= ilevel) break;
+      down(l);
+    }
   }
 
   // back substitution, new transports, layer sums of hydro_zeta
   double dbb = 0., dcb = 0., uold = 0., vold = 0., uh = 0., vh = 0.;
   float x0 = 0.f, x1 = 0.f, x2 = 0.f;
   float2 y0 = make_float2(0.f, 0.f), y1 = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int l = L - 1; l >= 0; l--) {
-    if (l >= NLV) continue;
+  auto up = [&](const int l) __attribute__((always_inline)) {
     const bool act = l < ilevel;
     float solu = 0.f, solv = 0.f, hre = 0.f, him = 0.f;
     if (act) {
       const bool blast = l == ilevel - 1;
       if constexpr (!COR) {
-        x0 = dp0[l] - (blast ? 0.f : cp[l] * x0);
-        x1 = dp1[l] - (blast ? 0.f : cp[l] * x1);
-        x2 = dp2[l] - (blast ? 0.f : cp[l] * x2);
+        const float c = SWEEP(cp, bC, l);
+        x0 = SWEEP(dp0, bP, l) - (blast ? 0.f : c * x0);
+        x1 = SWEEP(dp1, bQ, l) - (blast ? 0.f : c * x1);
+        x2 = SWEEP(dp2, bH, l) - (blast ? 0.f : c * x2);
         solu = x0; solv = x1; hre = x2;
       } else {
         if (blast) { y0 = dq0[l]; y1 = dq1[l]; }
@@ -347,9 +389,30 @@ __global__ void __launch_bounds__(128, W ? (XT ? 4 : 6) : 3) k_column_t(Dev d) {
       uold += (double)ul; vold += (double)vl;
       uh += (double)uhat; vh += (double)vhat;
     }
+  };
+  if constexpr (BIG) {
+#pragma unroll 1
+    for (int l = NLV - 1; l >= 0; l--) up(l);
+  } else {
+#pragma unroll
+    for (int l = L - 1; l >= 0; l--) {
+      if (l >= NLV) continue;
+      up(l);
+    }
   }
 
-  if constexpr (W) {
+  if constexpr (BIG) {
+    __syncwarp();
+    const size_t base = (size_t)w0 * NLV;
+#pragma unroll 4
+    for (int c = 0; c < nw; c++)
+      if (lane < NLV) {
+        const size_t q = base + (size_t)c * NLV + lane;
+        d.un[q] = bU[c * LS + lane];
+        d.vn[q] = bV[c * LS + lane];
+        d.ddx[q] = bH[c * LS + lane];
+      }
+  } else if constexpr (W) {
     __syncwarp();
     const size_t base = (size_t)w0 * NLV;
     const int cnt = nw * NLV;
@@ -400,6 +463,7 @@ __global__ void __launch_bounds__(128, W ? (XT ? 4 : 6) : 3) k_column_t(Dev d) {
 #undef COL_H
 #undef COL_U
 #undef COL_V
+#undef SWEEP
 }
 
 }  // namespace shy

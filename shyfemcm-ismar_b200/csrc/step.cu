@@ -75,12 +75,26 @@ static void launch_column_t(const Dev &d, cudaStream_t st, bool cor) {
   } else k_column_t<L, false, false><<<blocks, 128, 0, st>>>(d);
 }
 
+// columns of 17 to 32 layers: one warp per CTA, its columns and the sweep's
+// coefficients in shared memory
+static void launch_column_long(const Dev &d, cudaStream_t st) {
+  const int blocks = (d.NEL + 31) / 32;
+  const size_t smem = sizeof(float) * 6 * 32 * (d.NLV | 1);
+  if (d.mom) k_column_t<32, false, true, true><<<blocks, 32, smem, st>>>(d);
+  else if (d.any_xt) k_column_t<32, false, false, true><<<blocks, 32, smem, st>>>(d);
+  else k_column_t<32, false, false, true, false><<<blocks, 32, smem, st>>>(d);
+}
+
 void launch_elem(const Dev &d, int which, int init_only, cudaStream_t st, bool cor) {
   const bool thr = (d.col_threads || d.any_wd) && d.NLV <= 16;
   if (which == 0 && thr) {
     if (d.NLV <= 8) launch_column_t<8>(d, st, cor);
     else if (d.NLV <= 12) launch_column_t<12>(d, st, cor);
     else launch_column_t<16>(d, st, cor);
+    return;
+  }
+  if (which == 0 && d.col_threads && !cor) {     // more than 16 layers, no Coriolis
+    launch_column_long(d, st);
     return;
   }
   if (which == 1 && thr) {
