@@ -102,13 +102,13 @@ TeamShape zeta_team_shape() {
   return TeamShape{kTeamNT * 4, kTeamNT, 8, std::min(team_capacity(kZetaSym), team_capacity(kZetaGen))};
 }
 TeamShape csr_team_shape() { return TeamShape{kTeamNT, 2 * kTeamNT, 26, team_capacity(kCsrGen)}; }
-// Rows a CTA gets: 1024 in basins of up to 40 shares, where a team's
-// latency matters (7k rows: 0.31 ms a solve on 7 CTAs, 0.38 ms on 4), 2048
-// in larger ones, where more members only make the exchange slower (250k
-// rows: 0.42 ms on 123, 0.66 ms on 245) and the ensemble's basins take turns
-// on the CTAs (64 basins: 2.8 ms against 3.2 ms).  It depends on the basin
-// alone, so that its bits do.
-int zeta_team_share(int nk) { return nk <= 40960 ? kTeamNT * 2 : kTeamNT * 4; }
+// Rows a CTA gets: 1024 in small basins, where a team's latency matters (7k
+// rows: 0.31 ms a solve on 7 CTAs, 0.38 ms on 4), 2048 in larger ones, where
+// more members only make the exchange slower (250k rows: 0.42 ms on 123
+// CTAs, 0.66 ms on 245) and many basins take turns on the CTAs (the 64-basin
+// ensemble: 2.8 ms with 2048 rows everywhere, 3.6 ms with 1024 up to 40k
+// rows).  It depends on the basin alone, so that its bits do.
+int zeta_team_share(int nk) { return nk <= 12288 ? kTeamNT * 2 : kTeamNT * 4; }
 long long zeta_team_spin_limit() { return kTeamSpinLimit; }
 
 size_t zeta_grid_stage_smem(bool c16) { return 128 + 2 * (size_t)stage_layout(c16 ? 16 : 32).bytes; }

@@ -30,11 +30,11 @@ def levels(case, n=3, **opts):
 
 
 # one thread's rows, one CTA's, the first row of the next; the last team of
-# small shares and the first of large ones (40960 rows); the widest one-hop
-# team of small shares (41 warps' worth of members is two polling warps) and
+# small shares and the first of large ones (12288 rows); a one-hop team of
+# 20 members, one polled by two warps (36 members) and
 # one wider than 128 members
-@pytest.mark.parametrize("nx,ny", [(3, 3), (19, 27), (57, 9), (32, 32), (41, 25), (205, 10), (33, 1000 // 33 + 34),
-                                   (256, 160), (257, 160), (514, 514)])
+@pytest.mark.parametrize("nx,ny", [(3, 3), (19, 27), (57, 9), (32, 32), (41, 25), (205, 10), (33, 64),
+                                   (128, 96), (129, 96), (360, 200), (514, 514)])
 def test_resident_solver_matches_streaming(nx, ny):
     case = basin(nx, ny)
     (za,), a = levels(case)
