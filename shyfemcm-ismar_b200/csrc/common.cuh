@@ -179,7 +179,9 @@ struct Dev {
   double *vol_node;           // [k]
   double *vbud_node;          // [k] FP64 volume budget: the initial volume plus dt times every
                               //     step's flow into the node column (element fluxes, discharge)
-  float *stab_node;           // [s*NKN + k]
+  double2 *red_part;          // [b*red_chunks + c] volume and budget of a chunk of nodes (k_reduce)
+  unsigned *red_cnt;          // [b] chunks summed so far in the running launch
+  int red_chunks;             // chunks of the largest basin
   int *imax;                  // largest transport sub-step count of the step (all basins)
   int *subj;                  // sub-step index of the device-driven sub-step loop
   unsigned long long *nsub_launched;   // transport launches made by that loop

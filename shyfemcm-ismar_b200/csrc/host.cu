@@ -1380,6 +1380,8 @@ extern "C" int shygpu_create(int32_t nbasin, const shy_basin *B, const shy_param
   d.col_threads = 1;
   d.col_staged = 1;
   d.node_prefetch = 0;     // measured slower on the ensemble (spills): 1.04 against 0.82 ms
+  d.red_chunks = 1;
+  for (int b = 0; b < nbasin; b++) d.red_chunks = std::max(d.red_chunks, reduce_chunks(B[b].nkn));
   d.any_wd = m->any_wd ? 1 : 0;
   d.any_tvd = m->any_tvd ? 1 : 0;
   d.any_tvdv = 0;
@@ -1421,7 +1423,7 @@ extern "C" int shygpu_create(int32_t nbasin, const shy_basin *B, const shy_param
       A.alloc(&d.ddxi, m->cor ? EL : 1) || A.alloc(&d.cbnd, NSC) || A.alloc(&d.vol_node, NKN) || A.alloc(&d.vbud_node, NKN) ||
       A.alloc(&d.scr0, nsc_max > 0 ? NSC : 1) || A.alloc(&d.scr1, nsc_max > 0 ? NSC : 1) ||
       A.alloc(&d.imax, 1) || A.alloc(&d.subj, 1) || A.alloc(&d.nsub_launched, 1) ||
-      A.alloc(&d.stab_node, 1))
+      A.alloc(&d.red_part, (size_t)nbasin * d.red_chunks) || A.alloc(&d.red_cnt, nbasin))
     return bail(SHY_ECAPACITY);
   if (m->any_wd && (A.alloc(&d.iweg, NEL) || A.alloc(&d.iwet, NEL) || A.alloc(&d.inod, NKN) ||
                     A.upload(&d.kfull, kfull)))
@@ -1639,7 +1641,7 @@ extern "C" int shygpu_set_state(shygpu_model *m, int32_t ib, const shy_state *s)
   }
   launch_elem(d, 1, 1, st, m->cor);
   launch_node(d, m->kbas, 0, 1, 0, st);
-  launch_reduce(d, m->nsub, 0, st);
+  launch_reduce(d, 0, st);
   if (m->nsc_max > 0) launch_node(d, m->kbas, 3, 0, 0, st);
   g_launches += 3 + (m->nsc_max > 0);
   CUDA_TRY(cudaStreamSynchronize(st));
@@ -1746,7 +1748,7 @@ static int enqueue_hydro(shygpu_model *m, const Dev &d) {
 // the sub-step loop)
 static void enqueue_scalar_head(shygpu_model *m, const Dev &d) {
   if (m->nsc_max > 0) launch_node(d, m->kbas, 1, 0, 0, m->stream);   // k_stab
-  launch_reduce(d, 0, 1, m->stream);
+  launch_reduce(d, 1, m->stream);
 }
 
 // one transport sub-step j (-1: the device's counter): the TVD node
@@ -2715,7 +2717,7 @@ extern "C" int shygpu_profile_steps(shygpu_model *m, int32_t nsteps, double *ms_
     launch_elem(d, 1, 0, m->stream, m->cor); kind[n] = 2; cudaEventRecord(ev[++n], m->stream);
     launch_node(d, m->kbas, 0, 0, 0, m->stream); kind[n] = 3; cudaEventRecord(ev[++n], m->stream);
     if (m->nsc_max > 0) { launch_node(d, m->kbas, 1, 0, 0, m->stream); kind[n] = 4; cudaEventRecord(ev[++n], m->stream); }
-    launch_reduce(d, 0, 1, m->stream); kind[n] = 5; cudaEventRecord(ev[++n], m->stream);
+    launch_reduce(d, 1, m->stream); kind[n] = 5; cudaEventRecord(ev[++n], m->stream);
     if (m->nsc_max > 0) {
       int imax = 0;
       CUDA_TRY(cudaMemcpyAsync(&imax, d.imax, sizeof(int), cudaMemcpyDeviceToHost, m->stream));

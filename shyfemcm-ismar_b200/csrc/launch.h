@@ -29,7 +29,8 @@ void launch_elem(const Dev &d, int which, int init_only, cudaStream_t st, bool c
 // 4 k_rho, 5 k_moment, 6 k_tvdgrad(j=a), 7 k_conz with conz3d_omp's source
 // terms (j=a, one scalar)
 void launch_node(const Dev &d, const int *kbas, int which, int a, int b, cudaStream_t st);
-void launch_reduce(const Dev &d, int nsub, int advance, cudaStream_t st);
+void launch_reduce(const Dev &d, int advance, cudaStream_t st);
+int reduce_chunks(int nk);         // its CTAs for a basin of nk nodes
 // wetting and drying: 0 set_dry at the step's start, 1 the initial state's
 // setweg(0) (and zenv from znv), 2 setznv; basin >= 0 limits 1 and 2 to it
 void launch_wetdry(const Dev &d, const int *kbas, int which, int basin, cudaStream_t st);
