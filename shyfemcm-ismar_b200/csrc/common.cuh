@@ -121,11 +121,11 @@ struct Dev {
   const float *cz_obs, *cz_tau, *cz_wsv;
   float *cz_load;
   float cz_robs, cz_wsink, cz_rload;
-  // the transport's element part, per element vertex and layer: cz_ef
-  // [((3e + ii) * nsc_max + s) * NLV + l] = 4aj (3 fl - hdif) of scalar s on
-  // concentrations shifted by vertex ii's, cz_ef1 [(3e + ii) * NLV + l] =
-  // 4aj 3 fl of a unit field (the horizontal flow into the vertex)
-  float *cz_ef, *cz_ef1;
+  // the transport's element part, a record of (nsc_max + 1) * NLV floats per
+  // element vertex: 4aj 3 fl of a unit field (the horizontal flow into the
+  // vertex), then 4aj (3 fl - hdif) of each scalar on concentrations shifted
+  // by the vertex's own
+  float *cz_ef;
   BasinPar *par;
   BasinOut *out;
   // mesh (static)

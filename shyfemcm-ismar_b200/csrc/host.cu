@@ -1430,7 +1430,7 @@ extern "C" int shygpu_create(int32_t nbasin, const shy_basin *B, const shy_param
     return bail(SHY_ECAPACITY);
   if (m->any_adv && A.alloc(&d.mom, (size_t)NKN * NLV)) return bail(SHY_ECAPACITY);
   if (m->any_tvd && A.alloc(&d.tgrad, (size_t)nsc_max * NKN * NLV)) return bail(SHY_ECAPACITY);
-  if (nsc_max > 0 && (A.alloc(&d.cz_ef, (size_t)3 * NEL * nsc_max * NLV) || A.alloc(&d.cz_ef1, (size_t)3 * NEL * NLV)))
+  if (nsc_max > 0 && A.alloc(&d.cz_ef, (size_t)3 * NEL * (nsc_max + 1) * NLV))
     return bail(SHY_ECAPACITY);
   if (any_up && A.upload(&d.tvdup, tvdup)) return bail(SHY_ECAPACITY);
   m->xy_h.resize((size_t)2 * NKN);
@@ -1991,8 +1991,7 @@ extern "C" int shygpu_conz3d(shygpu_model *m, int32_t ib, float *cn1, float *co1
         A.alloc(&m->cz_cb, SN))
       return SHY_ECAPACITY;
     // the element part's buffers, for a model that transports nothing itself
-    if (!m->base.cz_ef && (A.alloc(&m->base.cz_ef, (size_t)3 * m->NEL * NLV) ||
-                           A.alloc(&m->base.cz_ef1, (size_t)3 * m->NEL * NLV)))
+    if (!m->base.cz_ef && A.alloc(&m->base.cz_ef, (size_t)6 * m->NEL * NLV))
       return SHY_ECAPACITY;
   }
   if (terms && !m->cz_obs) {

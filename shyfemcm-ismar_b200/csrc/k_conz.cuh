@@ -33,6 +33,8 @@
 // stays at the rounding of the stored values.
 // Included by node_launch.cuh.
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 #include "physics.cuh"
 
@@ -201,9 +203,10 @@ __global__ void __launch_bounds__(256) k_conz_el(Dev d, int j_arg) {
   for (int s = 0; s < nsc; s++) any |= isact <= (int)O.stab[s];
   if (!any) return;
   const bool act = lane < d.ilhv[e];
-  const size_t oe = (size_t)e * NLV + lane, e3 = (size_t)e * 3;
+  const size_t oe = (size_t)e * NLV + lane;
   const size_t SN = (size_t)d.NKN * NLV;
-  const int NSCM = d.nsc_max;
+  const int rl = (d.nsc_max + 1) * NLV;        // a vertex's record: the unit field's flux, then the scalars'
+  float *rec = d.cz_ef + (size_t)(unsigned)(3 * e) * (unsigned)rl + lane;
   const float4 e0 = *reinterpret_cast<const float4 *>(d.ev8 + (size_t)e * 8);
   const float4 e1 = *reinterpret_cast<const float4 *>(d.ev8 + (size_t)e * 8 + 4);
   const float bb[3] = {e0.x, e0.y, e0.z}, cc[3] = {e0.w, e1.x, e1.y};
@@ -222,7 +225,7 @@ __global__ void __launch_bounds__(256) k_conz_el(Dev d, int j_arg) {
   for (int ii = 0; ii < 3; ii++) {
     const float fii = f3[ii];
     const float fl1 = itot == 1 ? fii : (itot == 2 ? ((ii == 5 - isum) ? fii - (f3[0] + f3[1] + f3[2]) : fii) : 0.f);
-    d.cz_ef1[(e3 + ii) * NLV + lane] = act ? aj4 * 3.f * fl1 : 0.f;
+    rec[ii * rl] = act ? aj4 * 3.f * fl1 : 0.f;
   }
   const int kv[3] = {en.x, en.y, en.z};
   // TVD (the instance for models where a basin uses it): not where a vertex
@@ -271,7 +274,7 @@ __global__ void __launch_bounds__(256) k_conz_el(Dev d, int j_arg) {
         for (int iii = 0; iii < 3; iii++) wdiff += d.wdif[(size_t)e * 9 + 3 * iii + ii] * c3s[iii];
         hdif = 3.f * rk * dfh * hmed * wdiff;
       }
-      d.cz_ef[((e3 + ii) * NSCM + s) * NLV + lane] = act ? aj4 * (3.f * fl - hdif) : 0.f;
+      rec[ii * rl + (s + 1) * NLV] = act ? aj4 * (3.f * fl - hdif) : 0.f;
     }
   }
 }
@@ -329,16 +332,12 @@ __global__ void __launch_bounds__(256) k_conz(Dev d, const int *kbas, int j_arg)
   const float qf = mflux_layer<S>(d, k, act, o, P.wetdry != 0);
   const int pbeg = d.inc_ptr[k], pend = d.inc_ptr[k + 1];
   const bool up_ok = lane > 0, dn_ok = lane + 1 < lmax;
-  while (todo) {
-    // a group: scalars with the sub-step count of the first pending one
-    const int s0 = __ffs(todo) - 1;
-    const int istot = (int)O.stab[s0];
-    int sidx[NR];
-    int nm = 0;
-#pragma unroll
-    for (int r = 0; r < NR; r++) sidx[r] = -1;
-    for (int s = s0; s < nsc && nm < NR; s++)
-      if ((todo >> s & 1u) && (int)O.stab[s] == istot) { sidx[nm++] = s; todo &= ~(1u << s); }
+  // one group of scalars with the same sub-step count: sidx[r], or (ALL) the
+  // NR scalars of the basin in order, whose places are then constants
+  auto group = [&](auto all, const int istot, const int (&sidx)[NR]) {
+    constexpr bool ALL = decltype(all)::value;
+    auto has = [&](int r) { return ALL || sidx[r] >= 0; };
+    auto sc = [&](int r) { return ALL ? r : sidx[r]; };
     const float rstot = istot;
     const float rso = (isact - 1) / rstot, rsn = isact / rstot, rsot = 1.f - rso, rsnt = 1.f - rsn;
     const float dt = (float)P.dt / rstot;
@@ -355,9 +354,9 @@ __global__ void __launch_bounds__(256) k_conz(Dev d, const int *kbas, int j_arg)
     float cl[NR], cm1[NR], cp1[NR], hs[NR];
 #pragma unroll
     for (int r = 0; r < NR; r++) {
-      const int s = sidx[r] < 0 ? 0 : sidx[r];
+      const int s = has(r) ? sc(r) : 0;
       const bool istmp = P.is_temp[s] != 0;
-      const float v = (act && sidx[r] >= 0) ? clipc(cin_base[s * SN + o], istmp) : 0.f;
+      const float v = (act && has(r)) ? clipc(cin_base[s * SN + o], istmp) : 0.f;
       cl[r] = v;
       cm1[r] = seg_up<S>(v, 1);
       cp1[r] = seg_down<S>(v, 1);
@@ -369,16 +368,16 @@ __global__ void __launch_bounds__(256) k_conz(Dev d, const int *kbas, int j_arg)
     // each incident element, summed in element order
     float hs1 = 0.f;
     if (act) {
-      const int NSCM = d.nsc_max;
+      const unsigned rl = (unsigned)(d.nsc_max + 1) * NLV;
 #pragma unroll 4
       for (int p = pbeg; p < pend; p++) {
         const int4 ix = __ldg(&d.incx[p]);   // element, vertex | layers, other two nodes
         if (lane >= (ix.y >> 2)) continue;
-        const size_t ev = (size_t)ix.x * 3 + (ix.y & 3);
-        hs1 += d.cz_ef1[ev * NLV + lane];
+        const float *rec = d.cz_ef + (size_t)(unsigned)(3 * ix.x + (ix.y & 3)) * rl + lane;
+        hs1 += rec[0];
 #pragma unroll
         for (int r = 0; r < NR; r++)
-          if (sidx[r] >= 0) hs[r] += d.cz_ef[(ev * NSCM + sidx[r]) * NLV + lane];
+          if (has(r)) hs[r] += rec[(sc(r) + 1) * NLV];
       }
     }
     // storage, vertical diffusion and vertical advection, summed over the
@@ -431,8 +430,8 @@ __global__ void __launch_bounds__(256) k_conz(Dev d, const int *kbas, int j_arg)
       float q = hs[r] - fw - fd - fi;
       // boundary mass flux (conz3d_nodes :805-813): an inflow brings the
       // boundary concentration, an outflow takes the node's own (no change)
-      if (qf > 0.f && sidx[r] >= 0) {
-        const float cb = d.cbnd[sidx[r] * SN + o];
+      if (qf > 0.f && has(r)) {
+        const float cb = d.cbnd[sc(r) * SN + o];
         q += qf * (cb - c);
       }
       if constexpr (EX)                               // nudging, summed over the elements
@@ -469,11 +468,31 @@ __global__ void __launch_bounds__(256) k_conz(Dev d, const int *kbas, int j_arg)
     }
 #pragma unroll
     for (int r = 0; r < NR; r++) {
-      if (sidx[r] < 0) continue;
-      const int s = sidx[r];
+      if (!has(r)) continue;
+      const int s = sc(r);
       float cf = act ? cl[r] + res[r] : 0.f;         // old value plus increment
       if (act && isbnd && !d.conz_free_bnd) cf = d.cbnd[s * SN + o];      // bndo_impbc
       if (valid && lane < NLV) cout_base[s * SN + o] = cf;
+    }
+  };
+  while (todo) {
+    // the scalars with the sub-step count of the first pending one
+    const int istot = (int)O.stab[__ffs(todo) - 1];
+    unsigned cand = 0;
+    for (int s = 0; s < nsc; s++)
+      if ((todo >> s & 1u) && (int)O.stab[s] == istot) cand |= 1u << s;
+    int sidx[NR];
+    if (nsc == NR && cand == (1u << NR) - 1u) {
+      todo = 0;
+      group(std::true_type{}, istot, sidx);
+    } else {
+#pragma unroll
+      for (int r = 0; r < NR; r++) {
+        sidx[r] = __ffs(cand) - 1;                    // -1: none left
+        todo &= ~(cand & (0u - cand));
+        cand &= cand - 1u;
+      }
+      group(std::false_type{}, istot, sidx);
     }
   }
 }
