@@ -201,35 +201,53 @@ __global__ void __launch_bounds__(256) k_final_t(Dev d, int init_only) {
 // nzadapt <= 1) the element thickness needs no FP64 adaptive-layer terms
 // and the kernel keeps 80 registers, six CTAs per SM.
 // ===========================================================================
+// L > 16: one warp per CTA, its buffers in dynamic shared memory at an odd
+// stride (no bank conflicts).  Against a warp segment per column (k_final):
+// 250k elements of 23 layers 357 -> 235 us, 40k of 20 layers 27 -> 20 us.
 template <int L, bool ZA = true>
-__global__ void __launch_bounds__(128, ZA ? 1 : 6) k_final_w(Dev d, int init_only) {
-  __shared__ float sb[4][5][32 * L];
+__global__ void __launch_bounds__(L > 16 ? 32 : 128, L > 16 ? 1 : (ZA ? 1 : 6)) k_final_w(Dev d, int init_only) {
+  constexpr bool BIG = L > 16;
+  constexpr int NWARP = BIG ? 1 : 4;
+  __shared__ float sb[BIG ? 1 : 4][BIG ? 1 : 5][BIG ? 1 : 32 * L];
+  extern __shared__ float fin_dyn[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int w0 = (blockIdx.x * 4 + warp) * 32;         // first element of this warp
+  const int w0 = (blockIdx.x * NWARP + warp) * 32;     // first element of this warp
   if (w0 >= d.NEL) return;                              // whole warps only
   const int nw = min(32, d.NEL - w0);
   const int NLV = d.NLV, cnt = nw * NLV;
   const size_t base = (size_t)w0 * NLV;
-  float *bA = sb[warp][0], *bU = sb[warp][1], *bV = sb[warp][2], *bUo = sb[warp][3], *bVo = sb[warp][4];
+  const int LS = BIG ? NLV | 1 : NLV;                   // stride of the columns in the buffers
+  auto buf = [&](int q) { return BIG ? fin_dyn + q * 32 * LS : sb[BIG ? 0 : warp][BIG ? 0 : q]; };
+  float *bA = buf(0), *bU = buf(1), *bV = buf(2), *bUo = buf(3), *bVo = buf(4);
+  // fn(place in the buffers, place in global memory) over the warp's columns
+  auto sweep = [&](auto fn) {
+    if constexpr (BIG) {
+#pragma unroll 4
+      for (int c = 0; c < nw; c++)
+        if (lane < NLV) fn(c * LS + lane, base + (size_t)c * NLV + lane);
+    } else {
+      for (int j = lane; j < cnt; j += 32) fn(j, base + j);
+    }
+  };
   const bool valid = lane < nw;
   const int e = w0 + (valid ? lane : 0);
   const int4 en = d.enode[e];
   const BasinPar &P = d.par[en.w];
   const int kn[3] = {en.x, en.y, en.z};
   const int ilevel = d.ilhv[e];
-  const int ol = lane * NLV;                            // this thread's column in the buffers
+  const int ol = lane * LS;                             // this thread's column in the buffers
   const float *evp = d.ev8 + (size_t)e * 8;
   double zn3[3];
 #pragma unroll
   for (int ii = 0; ii < 3; ii++) zn3[ii] = d.zn[kn[ii]];
   if (!init_only) {
-    for (int j = lane; j < cnt; j += 32) {
-      bA[j] = d.ddx[base + j];
-      bU[j] = d.un[base + j];
-      bV[j] = d.vn[base + j];
-      bUo[j] = d.uo[base + j];
-      bVo[j] = d.vo[base + j];
-    }
+    sweep([&](int j, size_t q) {
+      bA[j] = d.ddx[q];
+      bU[j] = d.un[q];
+      bV[j] = d.vn[q];
+      bUo[j] = d.uo[q];
+      bVo[j] = d.vo[q];
+    });
     __syncwarp();
     if (valid) {
       const double beta = P.dt * (double)P.grav * P.am;
@@ -263,12 +281,12 @@ __global__ void __launch_bounds__(128, ZA ? 1 : 6) k_final_w(Dev d, int init_onl
       d.vnv[e] = (float)vm;
     }
     __syncwarp();
-    for (int j = lane; j < cnt; j += 32) {
-      d.un[base + j] = bU[j];
-      d.vn[base + j] = bV[j];
-      d.usv[base + j] = bUo[j];
-      d.vsv[base + j] = bVo[j];
-    }
+    sweep([&](int j, size_t q) {
+      d.un[q] = bU[j];
+      d.vn[q] = bV[j];
+      d.usv[q] = bUo[j];
+      d.vsv[q] = bVo[j];
+    });
     __syncwarp();
   }
   // setzev and the element part of setdepth (z-layers or pure sigma layers)
@@ -298,7 +316,7 @@ __global__ void __launch_bounds__(128, ZA ? 1 : 6) k_final_w(Dev d, int init_onl
     if (bad) set_status(&d.out[en.w], SHY_EDEPTH);
   }
   __syncwarp();
-  for (int j = lane; j < cnt; j += 32) d.hen[base + j] = bA[j];
+  sweep([&](int j, size_t q) { d.hen[q] = bA[j]; });
 }
 
 }  // namespace shy

@@ -5,15 +5,13 @@
 //             (hydrodynamic.f90:758-864, 868-1416, 488-733): one warp segment per
 //             element column, vertical system by PCR across lanes, 3x3 element
 //             system of the zeta equation written per element; k_column_t, the
-//             same with one thread per column (Thomas sweep) for columns of at
-//             most 16 layers.
+//             same with one thread per column (Thomas sweep).
 //   k_zeta    system_init/assemble/add_rhs/solve/get (simsys_spkaux.f90:137-705,
-//             sparskit_admin.f90:115-334): one thread-block cluster per basin;
-//             atomic-free gather assembly into CSR in element order (FP64), then
-//             FP32 preconditioned Krylov iterations inside FP64 residual
-//             refinement, all in one persistent launch.  k_zeta_grid does the
-//             same for basins too large for a cluster: one cooperative launch
-//             over the whole device.
+//             sparskit_admin.f90:115-334): atomic-free gather assembly in
+//             element order (FP64), then FP32 preconditioned Krylov
+//             iterations inside FP64 residual refinement, all in one
+//             persistent launch; the rows resident on chip (k_zeta_team),
+//             streamed (k_zeta_grid) or one cluster per basin (k_zeta).
 //   k_final   hydro_transports_final + setzev + element part of setdepth
 //             (hydrodynamic.f90:1468-1578, wetdry.f90:594, elems_dealing.f90:1063-1097).
 //   k_node    nodal part of setdepth + hydro_vertical + per-node volume
@@ -85,6 +83,13 @@ static void launch_column_long(const Dev &d, cudaStream_t st) {
   else k_column_t<32, false, false, true, false><<<blocks, 32, smem, st>>>(d);
 }
 
+static void launch_final_long(const Dev &d, int init_only, cudaStream_t st) {
+  const int blocks = (d.NEL + 31) / 32;
+  const size_t smem = sizeof(float) * 5 * 32 * (d.NLV | 1);
+  if (d.any_zad) k_final_w<32><<<blocks, 32, smem, st>>>(d, init_only);
+  else k_final_w<32, false><<<blocks, 32, smem, st>>>(d, init_only);
+}
+
 void launch_elem(const Dev &d, int which, int init_only, cudaStream_t st, bool cor) {
   const bool thr = (d.col_threads || d.any_wd) && d.NLV <= 16;
   if (which == 0 && thr) {
@@ -93,8 +98,9 @@ void launch_elem(const Dev &d, int which, int init_only, cudaStream_t st, bool c
     else launch_column_t<16>(d, st, cor);
     return;
   }
-  if (which == 0 && d.col_threads && !cor) {     // more than 16 layers, no Coriolis
-    launch_column_long(d, st);
+  if (d.col_threads && !cor && !thr) {           // more than 16 layers, no Coriolis
+    if (which == 0) launch_column_long(d, st);
+    else launch_final_long(d, init_only, st);
     return;
   }
   if (which == 1 && thr) {

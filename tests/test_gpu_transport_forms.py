@@ -105,3 +105,31 @@ def test_scalars_with_their_own_substep_counts():
     assert ns > nt and nb == ns
     assert np.abs(both["saltv"] - only_s["saltv"]).max() <= 1.0e-6 * np.abs(both["saltv"]).max()
     assert np.abs(both["tempv"] - only_t["tempv"]).max() <= 1.0e-6 * np.abs(both["tempv"]).max()
+
+
+@pytest.mark.parametrize("make,nlv,over", [
+    ("lagoon", 32, {}), ("basin3d", 17, {}), ("basin3d", 20, dict(nzadapt=3, ibarcl=0)), ("basin3d", 32, dict(nzadapt=32, ibarcl=0)),
+    ("hybrid", 26, {})])
+def test_long_columns_final_state_by_thread(make, nlv, over):
+    """Thickness, levels and transports after the zeta solve of columns of
+    17 to 32 layers (sigma, z, hybrid, z-adaptive) by a thread per column
+    against a warp segment per column, from the same start: the level of the
+    two runs differs by FP32 rounding, so thickness and transports agree to
+    1e-5 of the largest."""
+    case = (cases.lagoon_case(nkn_target=500, nlv=nlv) if make == "lagoon" else
+            cases.hybrid_lagoon_case(nkn_target=500, nsigma=nlv - 8) if make == "hybrid" else
+            cases.basin3d_case(nkn_target=700, nlv=nlv))
+    assert 16 < case["nlv"] <= 32
+    out = []
+    for threads in (1, 0):
+        m = shygpu.Model(case, **over)
+        m.set_option("column_threads", threads)
+        m.set_state_all()
+        m.run(2)
+        out.append(m.get_state(0))
+    for f in ("utlnv", "vtlnv", "hdknv", "hdenv"):
+        scale = np.abs(out[1][f]).max()
+        if f in ("utlnv", "vtlnv"):
+            scale = max(np.abs(out[1]["utlnv"]).max(), np.abs(out[1]["vtlnv"]).max())
+        assert np.abs(out[0][f] - out[1][f]).max() <= 1.0e-5 * scale, f
+    assert np.abs(out[0]["znv"] - out[1]["znv"]).max() <= 1.0e-5
