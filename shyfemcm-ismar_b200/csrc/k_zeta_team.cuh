@@ -589,11 +589,13 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
 #pragma unroll
         for (int r = 0; r < R; r++) { v[0] += (double)rr[r] * rr[r]; v[1] += (double)w[r] * rr[r]; }
         // 1 / gamma and 1 / alpha are kept, so that beta = g / gamma and alpha
-        // = g / (delta - beta g / alpha) wait for one division
+        // = g / (delta - beta g / alpha) wait for one reciprocal; a correctly
+        // rounded one is shorter than a division (per solve: 7k rows 330 ->
+        // 315 us, 793 rows 105.7 -> 102.6 us, 250k rows 428 -> 417 us)
         if (!exchange(w, gw, v, [&](const double (&t)[2]) {
               sh.fa = (float)(t[0] / t[1]);
               sh.fb = 0.f;
-              sh.rgamma = 1. / t[0];
+              sh.rgamma = __drcp_rn(t[0]);
               sh.ralpha = t[1] * sh.rgamma;
             })) { dead = true; break; }
         for (int inner = 1;; inner++) {
@@ -622,10 +624,10 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
           for (int r = 0; r < R; r++) { v[0] += (double)rr[r] * rr[r]; v[1] += (double)w[r] * rr[r]; }
           if (!exchange(w, gw, v, [&](const double (&t)[2]) {
                 const double beta = t[0] * sh.rgamma, den = t[1] - beta * t[0] * sh.ralpha;
-                sh.fa = (float)(t[0] / den);
+                sh.fa = (float)(t[0] * __drcp_rn(den));
                 sh.fb = (float)beta;
                 sh.stop = !(t[0] > sh.itol2) || !(t[0] == t[0]) || inner >= P.maxit;
-                sh.rgamma = 1. / t[0];
+                sh.rgamma = __drcp_rn(t[0]);
                 sh.ralpha = den * sh.rgamma;
               })) { dead = true; break; }
           iters++;
