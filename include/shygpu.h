@@ -381,7 +381,8 @@ int shygpu_set_bound_scalar(shygpu_model *model, int32_t ibasin, int32_t what,
  * fraction of the outer target, default 0.75), "max_outer" (FP64
  * refinement sweeps), "symmetric" (CG instead of BiCGStab; refused when
  * Coriolis makes the system non-symmetric), "column_threads" (1 one thread
- * per element column for up to 16 layers, 0 one warp segment),
+ * per element column (with Coriolis for up to 16 layers), 0 one warp
+ * segment),
  * "zeta_tile_rows" (rows per tile of the streaming solver, default 1024;
  * another value selects it),
  * "zeta_barrier_timeout_test" (failure detection: the device-wide solve's

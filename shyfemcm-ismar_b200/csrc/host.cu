@@ -1449,7 +1449,6 @@ extern "C" int shygpu_create(int32_t nbasin, const shy_basin *B, const shy_param
   }
   if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess)
     return bail(fail(SHY_ECUDA, "stream creation failed"));
-  // zeta solver launch shape: one cluster per basin, about 2k rows per CTA
   m->rowptr_h = rowptr;
   m->col_h = col;
   if (cudaEventCreateWithFlags(&m->ev_fork, cudaEventDisableTiming) != cudaSuccess)
@@ -1530,7 +1529,7 @@ extern "C" int shygpu_set_option(shygpu_model *m, const char *name, double value
       return st;
     }
   }
-  else if (n == "column_threads") {   // 1: one thread per column when it has at most 16 layers
+  else if (n == "column_threads") {   // 1: one thread per column (Coriolis: up to 16 layers)
     m->base.col_threads = iv != 0;
   }
   else if (n == "column_staged") {    // thread-per-column kernel: 1 columns staged in shared memory

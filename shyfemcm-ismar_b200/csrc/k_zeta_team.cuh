@@ -35,10 +35,12 @@
 // a number that is waited for.
 //
 // Measured (a solve, CUDA events; before: shared-memory clusters up to 40k
-// rows, the streaming solver above): 793 rows 51 iterations 268 -> 107 us,
-// 7k rows 121 iterations 615 -> 325 us, 20k rows 636 -> 315 us, 90k rows
-// 1156 -> 524 us, 250k rows 1139 -> 413 us, the 64-basin ensemble (2.1M rows)
-// 5.05 -> 2.77 ms.  What is left of an iteration (2 to 4 us) is a chain of
+// rows, the streaming solver above): 793 rows 51 iterations 268 -> 103 us,
+// 7k rows 121 iterations 615 -> 315 us, 20k rows 636 -> 360 us, 90k rows
+// 1156 -> 522 us, 250k rows 1139 -> 415 us, the 64-basin ensemble (2.1M rows)
+// 5.05 -> 2.71 ms; BiCGStab, 12k rows with Coriolis, 55 iterations 2.65 ->
+// 0.35 ms; the non-hydrostatic pressure (14k rows of up to 26 entries) 60 ->
+// 7 us an iteration.  What is left of an iteration (2 to 4 us) is a chain of
 // latencies: the gathers 0.5 us, the sums in the CTA and the FP64 scalars
 // 0.6 us, one exchange through L2 0.5 us for a few members, 1 us for many.
 //
@@ -563,7 +565,13 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
       if (sh.rn <= sh.tol || outer >= za.max_outer || (CSR && iters >= P.maxit)) break;
       if (tid == 0) {
         // the FP32 sweep's target, moved into the norm of the residual it works on
-        const double it0 = fmax((double)za.inner_rtol * sh.rn, tfrac(za) * sh.tol);
+        // (CG goes a tenth as far again: the iterations are the same in all, one
+        // refinement of three falls away, 7k rows 331 -> 318 us, 250k rows 428
+        // -> 405 us, and the level is closer to the exact one: the temperature
+        // of the 20k-node basin after 240 steps is 8.0e-5 from the oracle's,
+        // where rounding alone moved it between 7.7e-5 and 1.1e-4.  BiCGStab
+        // gains nothing: 12k rows 352 -> 376 us.)
+        const double it0 = fmax((SYM ? 0.1 : 1.) * (double)za.inner_rtol * sh.rn, tfrac(za) * sh.tol);
         sh.itol2 = sh.rn2 > 0. ? it0 * it0 * (sh.rs2 / sh.rn2) : 0.;
       }
       float e[R], ge[GR];                        // the correction
