@@ -216,19 +216,43 @@ static std::vector<T> padded(const std::vector<T> &v, size_t extra, T fill) {
 }
 
 struct Arena {
-  std::vector<void *> ptrs;
-  std::vector<size_t> sizes;         // bytes of each allocation (checkpoints)
-  int64_t bytes = 0;
+  std::vector<void *> ptrs;          // null: a place of the checkpoint format that holds nothing
+  std::vector<size_t> sizes;         // bytes of each place (checkpoints)
+  std::vector<void *> work;          // arrays that no launch reads before it has written them
+  int64_t bytes = 0;                 // of a checkpoint's places
+  int64_t held = 0;                  // on the device
   template <typename T>
-  int alloc(T **p, size_t n) {
+  int make(T **p, size_t n) {
     *p = nullptr;
-    if (n == 0) n = 1;
     cudaError_t e = cudaMalloc((void **)p, n * sizeof(T));
     if (e != cudaSuccess) return fail(SHY_ECAPACITY, "cudaMalloc of %zu bytes failed: %s", n * sizeof(T), cudaGetErrorString(e));
     cudaMemset(*p, 0, n * sizeof(T));
-    ptrs.push_back(*p);
-    sizes.push_back(n * sizeof(T));
-    bytes += (int64_t)(n * sizeof(T));
+    held += (int64_t)(n * sizeof(T));
+    return SHY_OK;
+  }
+  void place(void *p, size_t size) {
+    ptrs.push_back(p);
+    sizes.push_back(size);
+    bytes += (int64_t)size;
+  }
+  template <typename T>
+  int alloc(T **p, size_t n) {
+    if (n == 0) n = 1;
+    int st = make(p, n);
+    if (st == SHY_OK) place(*p, n * sizeof(T));
+    return st;
+  }
+  // outside of checkpoints
+  template <typename T>
+  int scratch(T **p, size_t n) {
+    int st = make(p, n);
+    if (st == SHY_OK) work.push_back(*p);
+    return st;
+  }
+  // the place in the checkpoint format of an array that is no longer kept
+  // (version 1 files stay readable, and their size as it was)
+  int hole(size_t size) {
+    place(nullptr, size);
     return SHY_OK;
   }
   template <typename T>
@@ -243,9 +267,11 @@ struct Arena {
   }
   void release() {
     for (void *p : ptrs) cudaFree(p);
+    for (void *p : work) cudaFree(p);
     ptrs.clear();
     sizes.clear();
-    bytes = 0;
+    work.clear();
+    bytes = held = 0;
   }
 };
 
@@ -898,7 +924,7 @@ extern "C" int64_t shygpu_footprint(int32_t nbasin, const shy_basin *basins, con
 }
 
 extern "C" int64_t shygpu_model_bytes(const shygpu_model *m) {
-  return m ? (int64_t)(m->arena.bytes + m->fstage_bytes) : -1;
+  return m ? (int64_t)(m->arena.held + m->fstage_bytes) : -1;
 }
 
 // the streams and events of the pipelined transfers, made on first use
@@ -1416,21 +1442,23 @@ extern "C" int shygpu_create(int32_t nbasin, const shy_basin *B, const shy_param
       A.alloc(&d.val32, nnz + 4) || A.alloc(&d.dinv32, NKN) || A.alloc(&d.r32, NKN) ||
       A.alloc(&d.p32, NKN) || A.alloc(&d.q32, NKN) || A.alloc(&d.z32, NKN) ||
       A.alloc(&d.e32, NKN) || A.alloc(&d.s32, NKN) || A.alloc(&d.t32, NKN) ||
-      A.alloc(&d.rh32, NKN) || A.alloc(&d.v32, NKN) ||
+      A.alloc(&d.rh32, NKN) || A.alloc(&d.v32, NKN) || A.hole(16 * (size_t)NKN) || A.hole(16 * (size_t)NKN) ||
+      A.hole(8 * ((size_t)NKN + 2)) ||
       A.alloc(&d.hia, (size_t)12 * NEL) || A.alloc(&d.unv, NEL) || A.alloc(&d.vnv, NEL) ||
       A.alloc(&d.usv, EL) || A.alloc(&d.vsv, EL) ||
       A.alloc(&d.wl, (size_t)NKN * (NLV + 1)) || A.alloc(&d.rho, NL) || A.alloc(&d.ddx, EL) ||
       A.alloc(&d.ddxi, m->cor ? EL : 1) || A.alloc(&d.cbnd, NSC) || A.alloc(&d.vol_node, NKN) || A.alloc(&d.vbud_node, NKN) ||
       A.alloc(&d.scr0, nsc_max > 0 ? NSC : 1) || A.alloc(&d.scr1, nsc_max > 0 ? NSC : 1) ||
       A.alloc(&d.imax, 1) || A.alloc(&d.subj, 1) || A.alloc(&d.nsub_launched, 1) ||
-      A.alloc(&d.red_part, (size_t)nbasin * d.red_chunks) || A.alloc(&d.red_cnt, nbasin))
+      A.hole(sizeof(float)) || A.scratch(&d.red_part, (size_t)nbasin * d.red_chunks) || A.scratch(&d.red_cnt, nbasin))
     return bail(SHY_ECAPACITY);
   if (m->any_wd && (A.alloc(&d.iweg, NEL) || A.alloc(&d.iwet, NEL) || A.alloc(&d.inod, NKN) ||
                     A.upload(&d.kfull, kfull)))
     return bail(SHY_ECAPACITY);
   if (m->any_adv && A.alloc(&d.mom, (size_t)NKN * NLV)) return bail(SHY_ECAPACITY);
   if (m->any_tvd && A.alloc(&d.tgrad, (size_t)nsc_max * NKN * NLV)) return bail(SHY_ECAPACITY);
-  if (nsc_max > 0 && A.alloc(&d.cz_ef, (size_t)3 * NEL * (nsc_max + 1) * NLV))
+  if (nsc_max > 0 && (A.scratch(&d.cz_ef, (size_t)3 * NEL * (nsc_max + 1) * NLV) ||
+                      A.hole(sizeof(float) * 3 * (size_t)NEL * nsc_max * NLV) || A.hole(sizeof(float) * 3 * EL)))
     return bail(SHY_ECAPACITY);
   if (any_up && A.upload(&d.tvdup, tvdup)) return bail(SHY_ECAPACITY);
   m->xy_h.resize((size_t)2 * NKN);
@@ -1995,7 +2023,8 @@ extern "C" int shygpu_conz3d(shygpu_model *m, int32_t ib, float *cn1, float *co1
         A.alloc(&m->cz_cb, SN))
       return SHY_ECAPACITY;
     // the element part's buffers, for a model that transports nothing itself
-    if (!m->base.cz_ef && A.alloc(&m->base.cz_ef, (size_t)6 * m->NEL * NLV))
+    if (!m->base.cz_ef && (A.scratch(&m->base.cz_ef, (size_t)6 * m->NEL * NLV) ||
+                           A.hole(sizeof(float) * 3 * (size_t)m->NEL * NLV) || A.hole(sizeof(float) * 3 * (size_t)m->NEL * NLV)))
       return SHY_ECAPACITY;
   }
   if (terms && !m->cz_obs) {
@@ -2105,7 +2134,8 @@ extern "C" int shygpu_checkpoint_save(shygpu_model *m, void *buf, int64_t nbytes
     p += sizeof sz;
   }
   for (size_t i = 0; i < m->arena.ptrs.size(); i++) {
-    CUDA_TRY(cudaMemcpy(p, m->arena.ptrs[i], m->arena.sizes[i], cudaMemcpyDeviceToHost));
+    if (m->arena.ptrs[i]) CUDA_TRY(cudaMemcpy(p, m->arena.ptrs[i], m->arena.sizes[i], cudaMemcpyDeviceToHost));
+    else memset(p, 0, m->arena.sizes[i]);
     p += m->arena.sizes[i];
   }
   return SHY_OK;
@@ -2135,7 +2165,7 @@ extern "C" int shygpu_checkpoint_load(shygpu_model *m, const void *buf, int64_t 
   }
   CUDA_TRY(cudaStreamSynchronize(m->stream));
   for (size_t i = 0; i < m->arena.ptrs.size(); i++) {
-    CUDA_TRY(cudaMemcpy(m->arena.ptrs[i], p, m->arena.sizes[i], cudaMemcpyHostToDevice));
+    if (m->arena.ptrs[i]) CUDA_TRY(cudaMemcpy(m->arena.ptrs[i], p, m->arena.sizes[i], cudaMemcpyHostToDevice));
     p += m->arena.sizes[i];
   }
   drop_graphs(m);

@@ -133,3 +133,31 @@ def test_long_columns_final_state_by_thread(make, nlv, over):
             scale = max(np.abs(out[1]["utlnv"]).max(), np.abs(out[1]["vtlnv"]).max())
         assert np.abs(out[0][f] - out[1][f]).max() <= 1.0e-5 * scale, f
     assert np.abs(out[0]["znv"] - out[1]["znv"]).max() <= 1.0e-5
+
+
+def test_checkpoint_keeps_the_places_of_version_1():
+    """A checkpoint holds the places of the arrays that version 1 had and the
+    model no longer keeps (zeros), whatever they hold on loading."""
+    case = cases.basin3d_case(nkn_target=700, nlv=20)
+    n, nel, nlv, nsc = case["nkn"], case["nel"], case["nlv"], 2
+    m = shygpu.Model(case)
+    m.set_state_all()
+    m.run(3)
+    ck = np.array(m.checkpoint(), copy=True).view(np.uint8)
+    count = int(ck[12:16].view(np.int32)[0])
+    sizes = ck[40:40 + 8 * count].view(np.int64)
+    start = 40 + 8 * count + np.r_[0, np.cumsum(sizes)]
+    assert start[-1] == ck.size
+    for gone in ([16 * n, 16 * n, 8 * (n + 2)], [12 * nel * nlv * nsc, 12 * nel * nlv]):
+        at = [i for i in range(count - len(gone) + 1) if list(sizes[i:i + len(gone)]) == gone]
+        assert len(at) == 1
+        a, b = start[at[0]], start[at[0] + len(gone)]
+        assert not ck[a:b].any()
+        ck[a:b] = 0x7f
+    m.run(3)
+    want = m.get_state(0)
+    m.restore(ck)
+    m.run(3)
+    got = m.get_state(0)
+    for f in ("znv", "utlnv", "tempv"):
+        assert np.array_equal(got[f], want[f]), f
