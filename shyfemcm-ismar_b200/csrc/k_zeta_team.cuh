@@ -339,11 +339,11 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
       const int i = ri[r] & 0x7fffffff;
       double diag = 0., tA, tB = 0.;
       if constexpr (CSR) {
-        diag = val64[rowptr[i] + (tp.dpos[M.row0 + j] & 0xff)];
+        diag = val64[rowptr[i] + dpos_place(tp.dpos[M.row0 + j])];
         tA = rhs64[i];                           // the guess is zero
       } else {
         const int s0 = d.rowptr[i];
-        const int dn = tp.dpos[M.row0 + j], dp = dn & 0xff, nd = dn >> 8;   // diagonal's place, off-diagonal entries
+        const int dn = tp.dpos[M.row0 + j], dp = dpos_place(dn), nd = dpos_count(dn);   // diagonal's place, off-diagonal entries
         double rhs = 0.;
         const int p1 = d.inc_ptr[i + 1];
         for (int p0 = d.inc_ptr[i]; p0 < p1; p0 += 8) {   // eight elements at a time, their loads in flight together
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
           col[r][k] = __ldg(reinterpret_cast<const unsigned *>(tp.lcol) + (size_t)(M.row0 + j) * (K / 2) + k);
       }
       const int i = ri[r] & 0x7fffffff;
-      const int dn = tp.dpos[M.row0 + j], dp = dn & 0xff, nd = dn >> 8;
+      const int dn = tp.dpos[M.row0 + j], dp = dpos_place(dn), nd = dpos_count(dn);
       const double sdi = SYM ? (double)sh.sd[j] : 1.;
       const double *a = val64 + rowptr[i];
 #pragma unroll
@@ -744,7 +744,7 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
         rr[r] = 0.f;
         if (j >= n) continue;
         const int i = ri[r] & 0x7fffffff;
-        const int dn = tp.dpos[M.row0 + j], dp = dn & 0xff, nd = dn >> 8;
+        const int dn = tp.dpos[M.row0 + j], dp = dpos_place(dn), nd = dpos_count(dn);
         const double *a = val64 + rowptr[i];
         double t = rhs64[i] - a[dp] * sh.x[j];
 #pragma unroll

@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "team_plan.h"
 
 namespace shy {
 
@@ -126,7 +127,7 @@ struct TeamMember {
 // one order of the basins common to all CTAs).  Per row of the shares, in
 // their order: the global row (sign bit: some other member holds a ghost of
 // it), the place of the diagonal among the row's CSR slots with the count
-// of the others (dpos: place | count << 8), and the share's local column
+// of the others (dpos: dpos_pack), and the share's local column
 // (own rows, from zeta_team_rows() on the ghosts) of the first eight off-diagonal entries (lcol, as
 // byte offsets into a float array; the row itself on padding); rows with more keep the rest in a tail (tptr,
 // tcol, tslot, tval; null when no row has one).  word: four exchange buffers
@@ -174,13 +175,6 @@ cudaError_t launch_zeta_grid(const Dev &d, const ZetaArgs &za, const GridPlan &g
 cudaError_t launch_zeta_team(const Dev &d, const ZetaArgs &za, const TeamPlan &tp, int G, cudaStream_t st);
 // its CSR instance: the systems of the 3D pressure
 cudaError_t launch_csr_team(const Dev &d, const ZetaArgs &za, const TeamPlan &tp, int G, cudaStream_t st);
-// what a CTA of the resident solver holds
-struct TeamShape {
-  int rows;      // rows at most (the first place of a ghost)
-  int ghosts;    // ghost copies at most
-  int entries;   // off-diagonal entries in a row's block
-  int capacity;  // CTAs that fit the device at once (0 on error)
-};
 TeamShape zeta_team_shape();
 TeamShape csr_team_shape();
 int zeta_team_share(int nk); // rows a CTA gets at most in a basin of nk rows

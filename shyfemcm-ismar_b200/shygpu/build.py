@@ -18,7 +18,7 @@ CSRC = PKG / "csrc"
 LIB = HERE / "libshygpu.so"
 SOURCES = ["step_node32.cu", "step_node16.cu", "step_zeta.cu", "step_node.cu", "step.cu", "host.cu",
            "static_solve.cu", "serve.cu", "nonhydro.cu"]
-HEADERS = ["common.cuh", "launch.h", "physics.cuh", "node_launch.cuh", "k_column.cuh", "k_column_t.cuh", "k_final.cuh", "k_node.cuh", "k_conz.cuh", "k_zeta.cuh", "k_wetdry.cuh", "k_zeta_global.cuh", "k_zeta_grid.cuh", "k_zeta_team.cuh"]
+HEADERS = ["common.cuh", "launch.h", "team_plan.h", "physics.cuh", "node_launch.cuh", "k_column.cuh", "k_column_t.cuh", "k_final.cuh", "k_node.cuh", "k_conz.cuh", "k_zeta.cuh", "k_wetdry.cuh", "k_zeta_global.cuh", "k_zeta_grid.cuh", "k_zeta_team.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -1,0 +1,96 @@
+"""Which zeta and pressure solver a model runs, and that each of them, and
+each way from one to the next, gives the same levels.
+
+Tolerances: a level against the oracle to the parity tolerance, 1e-3 m;
+levels of two solvers, which both end on ||r|| <= 1e-8 ||r0|| + 1e-8 in FP64,
+to 1e-5 m on regular meshes and 1e-4 m on discs whose elements are fifty
+times longer than wide; pressures to 1e-2 of the largest, the tolerance of
+the non-hydrostatic parity tests."""
+import numpy as np
+import pytest
+
+import shygpu
+import shyref
+from shygpu import cases
+
+pytestmark = pytest.mark.gpu
+
+ZETA_TOL = 1.0e-3
+
+
+def disc(spokes, rings=4, r0=400.0, dr=100.0, nlv=1, depth=10.0, level=None, **params):
+    """Rings of `spokes` nodes around a hub, which is numbered last (its
+    neighbours all come before it); one layer with the tide on the outer
+    ring, or `nlv` sigma layers, closed, from the start level `level`."""
+    ang = 2 * np.pi * np.arange(spokes) / spokes
+    rad = r0 + dr * np.arange(rings)
+    x = np.r_[(rad[:, None] * np.cos(ang)).ravel(), 0.0]
+    y = np.r_[(rad[:, None] * np.sin(ang)).ravel(), 0.0]
+    hub = rings * spokes
+    node = lambda r, s: r * spokes + s % spokes
+    tri = [(hub, node(0, s), node(0, s + 1)) for s in range(spokes)]
+    for r in range(rings - 1):
+        for s in range(spokes):
+            tri += [(node(r, s), node(r + 1, s), node(r + 1, s + 1)), (node(r, s), node(r + 1, s + 1), node(r, s + 1))]
+    nen = np.asarray(tri, np.int32) + 1
+    nkn, nel = len(x), len(tri)
+    hk = depth * (1.0 + 0.1 * np.sin(x / rad[-1] * 2.0))
+    c = cases.channel_case(nx=3, ny=3)
+    for k in ("czv", "fcorv", "visv", "difv", "tauxnv", "tauynv", "ppv", "rqv", "znv", "utlnv", "vtlnv", "tempv",
+              "saltv", "conzv"):
+        c.pop(k, None)
+    bnd = np.zeros(nkn, np.int32)
+    if level is None:
+        bnd[node(rings - 1, 0):hub] = 1
+    else:
+        c["tide"] = np.zeros((0, 1, 4), np.float32)
+        c["znv"] = (level * np.cos(np.pi * x / (2 * rad[-1]))).astype(np.float32)
+        c["params"] = dict(c["params"], ireib=0)
+    if nlv > 1:
+        c.update(hlv=-np.arange(1, nlv + 1) / nlv, hldv=np.full(nlv, -1.0 / nlv))
+        c["params"] = dict(c["params"], nsigma=nlv)
+    c.update(name="disc", nkn=nkn, nel=nel, nlv=nlv, nen3v=nen, xgv=x, ygv=y, hm3v=hk[nen - 1],
+             ilhv=np.full(nel, nlv, np.int32), ilhkv=np.full(nkn, nlv, np.int32), bnd_index=bnd,
+             params=dict(c["params"], **params))
+    return cases._finish(c)
+
+
+def nh_disc(spokes):
+    return disc(spokes, r0=40.0, dr=10.0, nlv=3, depth=15.0, level=0.01, dt=0.2, inohyd=1)
+
+
+def run(case, n, **opts):
+    m = shygpu.Model(case)
+    for k, v in opts.items():
+        m.set_option(k, v)
+    m.set_state_all()
+    m.run(n)
+    return m
+
+
+def znv(m, i=0):
+    return m.get_state(i, ("znv",))["znv"]
+
+
+@pytest.mark.parametrize("spokes", [255, 256, 300])
+def test_hub_of_more_than_255_neighbours(spokes):
+    """The hub's diagonal is the last of its row's entries."""
+    c = disc(spokes)
+    a, b = run(c, 10), run(c, 10, zeta_tile_rows=512)
+    o = shyref.OracleModel(c)
+    o.run(10)
+    assert np.abs(znv(a) - o.state()["znv"]).max() <= ZETA_TOL
+    assert np.abs(znv(a) - znv(b)).max() <= 1.0e-4
+
+
+@pytest.mark.parametrize("spokes", [250, 300])
+def test_pressure_of_a_hub_of_more_than_255_neighbours(spokes):
+    c = nh_disc(spokes)
+    g = run(c, 5)
+    o = shyref.OracleModel(c)
+    o.run(5)
+    assert np.abs(znv(g) - o.state()["znv"]).max() <= 1.0e-3 * 0.01
+    q, (it, _, r0, r) = g.nh(0)
+    qo = o.nh()[0]
+    assert it > 0 and r <= 1e-8 * r0 + 1e-8
+    assert np.abs(q - qo).max() <= 1.0e-2 * np.abs(qo).max()
