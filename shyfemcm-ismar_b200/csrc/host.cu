@@ -371,6 +371,14 @@ static void drop_graphs(shygpu_model *m) {
 
 static int check_cluster_shape(int CL, int threads);
 
+// Ends the default stream's zeroing and copies.  cudaMemset does not wait for
+// the device, and the models' streams do not wait for the default stream, so
+// an array zeroed there may be cleared after a launch has written it.
+static int settle() {
+  CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+  return SHY_OK;
+}
+
 // Zeta launch plan.  A model runs in one cooperative launch over the device:
 // the resident solver (k_zeta_team), or, when a basin does not fit on chip
 // or its tiles are asked for, the streaming one (k_zeta_grid) if the system
@@ -715,7 +723,8 @@ static int build_zeta_plan_impl(shygpu_model *m, int forceCL, int forceThreads);
 // forceCL > 0: one class with that shape for every basin.  A plan that
 // cannot be built leaves no plan (the step then refuses to run).
 static int build_zeta_plan(shygpu_model *m, int forceCL, int forceThreads) {
-  const int st = build_zeta_plan_impl(m, forceCL, forceThreads);
+  int st = build_zeta_plan_impl(m, forceCL, forceThreads);
+  if (st == SHY_OK) st = settle();
   if (st != SHY_OK) free_zeta_plan(m);
   return st;
 }
@@ -1942,6 +1951,7 @@ extern "C" int shygpu_conz3d(shygpu_model *m, int32_t ib, float *cn1, float *co1
     if (!m->base.cz_ef && (A.scratch(&m->base.cz_ef, (size_t)6 * m->NEL * NLV) ||
                            A.hole(sizeof(float) * 3 * (size_t)m->NEL * NLV) || A.hole(sizeof(float) * 3 * (size_t)m->NEL * NLV)))
       return SHY_ECAPACITY;
+    ST_TRY(settle());
   }
   if (terms && !m->cz_obs) {
     CUDA_TRY(cudaStreamSynchronize(st));
@@ -1949,6 +1959,7 @@ extern "C" int shygpu_conz3d(shygpu_model *m, int32_t ib, float *cn1, float *co1
     if (A.alloc(&m->cz_obs, SN) || A.alloc(&m->cz_tau, SN) || A.alloc(&m->cz_load, SN) ||
         A.alloc(&m->cz_wsv, (size_t)m->NKN * (NLV + 1)))
       return SHY_ECAPACITY;
+    ST_TRY(settle());
   }
   // the sub-step's parameters: basin ib transports one scalar, unclipped
   // (scal3sh clips before the call), the others nothing
@@ -2084,6 +2095,7 @@ extern "C" int shygpu_checkpoint_load(shygpu_model *m, const void *buf, int64_t 
     if (m->arena.ptrs[i]) CUDA_TRY(cudaMemcpy(m->arena.ptrs[i], p, m->arena.sizes[i], cudaMemcpyHostToDevice));
     p += m->arena.sizes[i];
   }
+  ST_TRY(settle());
   drop_graphs(m);
   m->cur = h.cur;
   m->sc_cur = h.sc_cur;
@@ -2614,6 +2626,7 @@ extern "C" int shygpu_set_nudging(shygpu_model *m, int32_t ib, const float *andg
   if (!m->base.andg) {             // first use: the array (zeros elsewhere) and new graphs that read it
     CUDA_TRY(cudaStreamSynchronize(m->stream));
     if (m->arena.alloc(&m->base.andg, (size_t)m->NKN)) return SHY_ECAPACITY;
+    ST_TRY(settle());
     drop_graphs(m);
   }
   CUDA_TRY(cudaMemcpyAsync(m->base.andg + bp.k0, andgzv, (size_t)bp.nk * 4, cudaMemcpyHostToDevice, m->stream));
@@ -3105,7 +3118,8 @@ static int simsys_init_impl() {
   if (!g_sys.st) CUDA_TRY(cudaStreamCreateWithFlags(&g_sys.st, cudaStreamNonBlocking));
   g_sys.initialized = true;
   g_sys.explicit_mode = false;
-  return simsys3d_init(pt);
+  ST_TRY(simsys3d_init(pt));
+  return settle();
 }
 
 extern "C" void system_initialize_(void) {           // simsys_spkaux.f90:85

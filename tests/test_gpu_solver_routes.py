@@ -94,3 +94,31 @@ def test_pressure_of_a_hub_of_more_than_255_neighbours(spokes):
     qo = o.nh()[0]
     assert it > 0 and r <= 1e-8 * r0 + 1e-8
     assert np.abs(q - qo).max() <= 1.0e-2 * np.abs(qo).max()
+
+
+@pytest.mark.parametrize("variant", [1, 0])
+@pytest.mark.parametrize("tile_rows", [0, 512])
+def test_plan_made_while_the_default_stream_is_busy(variant, tile_rows):
+    """A plan starts from zeroed words and counters whatever another part of
+    the program has queued on the default stream meanwhile."""
+    import threading
+    import torch
+
+    c = cases.channel_case(nx=120, ny=60, lx=150.0 * 119, ly=150.0 * 59)
+    want = znv(run(c, 6, zeta_variant=variant, zeta_tile_rows=tile_rows))
+    m = shygpu.Model(c)
+    m.set_state_all()
+    torch.cuda.synchronize()
+
+    def busy():
+        for _ in range(60):
+            torch.cuda._sleep(8_000_000)                     # 4 ms each, a quarter of a second in all
+    t = threading.Thread(target=busy)
+    t.start()
+    for _ in range(3):
+        m.set_option("zeta_variant", variant)
+        m.set_option("zeta_tile_rows", tile_rows)
+        m.run(2)
+    t.join()
+    torch.cuda.synchronize()
+    assert np.array_equal(znv(m), want)
