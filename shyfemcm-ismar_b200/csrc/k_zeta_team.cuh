@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
     if (!CSR && M.rank == 0 && tid < kMaxScal) O.stab[tid] = 0.f;   // reset for k_stab's max
     const float dtf = (float)P.dt;
     // wetting and drying: a domain that can change with the solution
-    const bool wd = !SYM && !CSR && wd_basin(P) && !za.explicit_mode;
+    const bool wd = !SYM && !CSR && wd_basin(P);
     const bool extrap = !CSR && za.zprev != nullptr && O.steps > 0 && !wd;
     // a barrier of the team that also makes its global writes visible; sums
     // one value
@@ -363,12 +363,6 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
         if (!(wd && d.inod[i] == -2)) rhs += (double)(dtf * d.rqv[i]);
         d.rhs64[i] = rhs;
         const double zg = level(i);
-        if (za.explicit_mode) {
-          const double x0 = diag != 0. ? rhs / diag : 0.;
-          d.x64[i] = x0;
-          d.zn[i] = (float)x0;
-          continue;
-        }
         d.val64[s0 + dp] = diag;
         tA = rhs - diag * zg;
         tB = extrap ? rhs - diag * (2. * zg - (double)za.zprev[i]) : 0.;
@@ -403,10 +397,6 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
       v4[1] += (double)rsA[r] * rsA[r];
       v4[2] += tB * tB;
       v4[3] += (double)rsB[r] * rsB[r];
-    }
-    if (za.explicit_mode) {                      // system_set_explicit: no coupling between rows
-      if (M.rank == 0 && tid == 0) { O.iters = 0; O.refinements = 0; O.resid0 = 0.; O.resid = 0.; }
-      break;
     }
     unsigned ep = number();
 #pragma unroll
@@ -785,7 +775,6 @@ __global__ void __launch_bounds__(NT, 1) k_zeta_team(Dev d, ZetaArgs za, TeamPla
     if (rep + 1 >= kWetDryRepeats) { if (M.rank == 0 && tid == 0) set_status(&O, SHY_ENOCONV); break; }
     }
     if (dead) break;
-    if (za.explicit_mode) continue;
     if (tid == 0 && M.rank == 0) {
       if constexpr (CSR) {
         O.nh_iters = iters;
