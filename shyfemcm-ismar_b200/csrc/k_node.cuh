@@ -437,24 +437,25 @@ __global__ void __launch_bounds__(256) k_stab(Dev d, const int *kbas) {
 
 // ===========================================================================
 // k_reduce: per basin volume, sub-step counts, time.  Chunks of kReduceChunk
-// nodes, one CTA each (blockIdx.x) of every basin (blockIdx.y); the CTA that
-// finishes a basin last adds the chunks' sums in order, so a basin's sums
-// depend on it alone.  One CTA per basin took 162 us on 250k nodes (the
+// nodes, one CTA each (blockIdx.y) of every basin (blockIdx.x: a grid has at
+// most 65535 CTAs in y); the CTA that finishes a basin last adds the chunks'
+// sums in order, so a basin's sums depend on it alone.  One CTA per basin took 162 us on 250k nodes (the
 // latency of 244 dependent loads a thread); the chunks take 33 us.
 // ===========================================================================
 constexpr int kReduceChunk = 4096;
 
 static __global__ void __launch_bounds__(1024) k_reduce(Dev d, int advance) {
-  const int b = blockIdx.y;
+  const int b = blockIdx.x;
   const BasinPar &P = d.par[b];
   const int nchunk = (P.nk + kReduceChunk - 1) / kReduceChunk;
-  if ((int)blockIdx.x >= nchunk) return;
+  const int chunk = blockIdx.y;
+  if (chunk >= nchunk) return;
   BasinOut &O = d.out[b];
   __shared__ double part[32], partb[32];
   __shared__ bool last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double s = 0., sb = 0.;
-  const int k0 = blockIdx.x * kReduceChunk, k1 = min(P.nk, k0 + kReduceChunk);
+  const int k0 = chunk * kReduceChunk, k1 = min(P.nk, k0 + kReduceChunk);
 #pragma unroll
   for (int q = 0; q < kReduceChunk / 1024; q++) {
     const int k = k0 + q * 1024 + tid;
@@ -473,7 +474,7 @@ static __global__ void __launch_bounds__(1024) k_reduce(Dev d, int advance) {
   cta_sum(s, sb);
   if (nchunk > 1) {
     if (tid == 0) {
-      d.red_part[(size_t)b * gridDim.x + blockIdx.x] = make_double2(s, sb);
+      d.red_part[(size_t)b * gridDim.y + chunk] = make_double2(s, sb);
       __threadfence();
       last = atomicAdd(&d.red_cnt[b], 1u) + 1u == (unsigned)nchunk;
       if (last) d.red_cnt[b] = 0u;               // for the next launch
@@ -483,7 +484,7 @@ static __global__ void __launch_bounds__(1024) k_reduce(Dev d, int advance) {
     __threadfence();
     s = sb = 0.;
     for (int c = tid; c < nchunk; c += 1024) {
-      const double2 v = __ldcg(&d.red_part[(size_t)b * gridDim.x + c]);
+      const double2 v = __ldcg(&d.red_part[(size_t)b * gridDim.y + c]);
       s += v.x; sb += v.y;
     }
     cta_sum(s, sb);

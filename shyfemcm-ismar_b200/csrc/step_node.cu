@@ -50,7 +50,7 @@ void launch_node(const Dev &d, const int *kbas, int which, int a, int b, cudaStr
 }
 
 void launch_reduce(const Dev &d, int advance, cudaStream_t st) {
-  k_reduce<<<dim3(d.red_chunks, d.nbasin), 1024, 0, st>>>(d, advance);
+  k_reduce<<<dim3(d.nbasin, d.red_chunks), 1024, 0, st>>>(d, advance);
 }
 
 int reduce_chunks(int nk) { return (nk + kReduceChunk - 1) / kReduceChunk; }

@@ -122,3 +122,16 @@ def test_plan_made_while_the_default_stream_is_busy(variant, tile_rows):
     t.join()
     torch.cuda.synchronize()
     assert np.array_equal(znv(m), want)
+
+
+def test_more_basins_than_a_grid_has_rows():
+    """65540 basins in one model (a grid has at most 65535 CTAs in y and z):
+    the sums over a basin, of the first, a middle and the last one."""
+    cs = [cases.channel_case(nx=3, ny=3, lx=300.0, ly=300.0, seed=s) for s in (1, 2)]
+    n = 65540
+    m = shygpu.Model([cs[0]] * (n - 1) + [cs[1]])
+    for i, c in ((0, cs[0]), (n // 2, cs[0]), (n - 1, cs[1])):
+        m.set_state(i)
+        a = shygpu.Model(c)
+        a.set_state(0)
+        assert a.info(0).volume == m.info(i).volume > 0
