@@ -31,8 +31,10 @@
 // uses three others).  Every wait is bounded; one that runs out sets the
 // abort word, marks the basins SHY_ECUDA and all CTAs leave.  The number of
 // an exchange is the launch's (16 bits) and its place in the launch (16
-// bits); every word is written in every launch, so an old one never carries
-// a number that is waited for.
+// bits).  A share's first exchange of a launch writes all its words, those
+// that only later exchanges carry included, so an old word never has a
+// number that is waited for: only 65536 launches in a row that were aborted
+// before they reached the share would bring it back.
 //
 // Measured (a solve, CUDA events; before: shared-memory clusters up to 40k
 // rows, the streaming solver above): 793 rows 51 iterations 268 -> 103 us,
@@ -137,9 +139,12 @@ __device__ __forceinline__ u64 *team_slot(const TeamPlan &tp, unsigned xi, int d
   return tp.part + (((size_t)(xi & 1u) * 2 + down) * tp.nslot + slot) * kTeamSlotWords;
 }
 
+constexpr int kTeamSums = 12;        // words of the widest exchange (three pairs)
+static_assert(kTeamSums <= kTeamSlotWords, "a slot holds them");
+
 // word k of a slot that holds the 2 NP sums x (every lane has them all) as
-// low and high halves; the first exchange of a launch renews the other
-// buffer's word too
+// low and high halves.  The first exchange of a launch renews both buffers'
+// words up to kTeamSums, whatever the exchanges that follow carry.
 template <int NP>
 __device__ __forceinline__ void sums_put(const TeamPlan &tp, unsigned xi, int down, int slot, const double (&x)[2 * NP],
                                          unsigned ep, int k) {
@@ -202,7 +207,7 @@ __device__ __forceinline__ bool team_totals(SH &sh, const TeamPlan &tp, const Te
       for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
       both_sums(x, tot[2 * c], tot[2 * c + 1]);
     }
-    if (T > 1 && lane < 4 * NP) sums_put<NP>(tp, xi, 0, M.slot0 + M.rank, tot, ep, lane);
+    if (T > 1 && lane < (xi == 0u ? kTeamSums : 4 * NP)) sums_put<NP>(tp, xi, 0, M.slot0 + M.rank, tot, ep, lane);
   }
   if (T == 1) return true;
   // nobody polls before warp 0 has published: the polls would queue ahead of its stores
@@ -224,9 +229,14 @@ __device__ __forceinline__ bool team_totals(SH &sh, const TeamPlan &tp, const Te
         for (int w = 1; w < nw; w++)
 #pragma unroll
           for (int c = 0; c < 2 * NP; c++) tot[c] += sh.tsum[c][w];
-        if (!all)
-          for (int k = lane; k < 4 * NP * M.T; k += 32)
-            sums_put<NP>(tp, xi, 1, M.slot0 + k / (4 * NP), tot, ep, k % (4 * NP));
+        if (!all) {
+          if (xi == 0u)
+            for (int k = lane; k < kTeamSums * M.T; k += 32)
+              sums_put<NP>(tp, xi, 1, M.slot0 + k / kTeamSums, tot, ep, k % kTeamSums);
+          else
+            for (int k = lane; k < 4 * NP * M.T; k += 32)
+              sums_put<NP>(tp, xi, 1, M.slot0 + k / (4 * NP), tot, ep, k % (4 * NP));
+        }
       }
     }
   } else if (warp == 0) {

@@ -135,3 +135,18 @@ def test_more_basins_than_a_grid_has_rows():
         a = shygpu.Model(c)
         a.set_state(0)
         assert a.info(0).volume == m.info(i).volume > 0
+
+
+def test_levels_across_the_wrap_of_the_launch_number():
+    """The resident solver numbers its launches with 16 bits: twelve steps
+    across the wrap give the levels that the cluster solver gives."""
+    c = cases.channel_case(nx=41, ny=25)
+    c["fcorv"] = np.full(c["nel"], 1.0e-4, np.float32)
+    m = run(c, 65530)
+    ck = m.checkpoint()
+    m.run(12)
+    a = znv(m)
+    m.restore(ck)
+    m.set_option("zeta_variant", 0)
+    m.run(12)
+    assert np.abs(a).max() > 0.01 and np.abs(a - znv(m)).max() <= 1.0e-5
