@@ -223,13 +223,14 @@ __device__ __forceinline__ bool team_totals(SH &sh, const TeamPlan &tp, const Te
         for (int c = 0; c < 2 * NP; c++) sh.tsum[c][warp] = tot[c];
     }
     if (T > 32) {                                  // uniform in the CTA
+      if (!ok) sh.ok = 0;
       __syncthreads();
       if (warp == 0) {
         const int nw = (T + 31) / 32;
         for (int w = 1; w < nw; w++)
 #pragma unroll
           for (int c = 0; c < 2 * NP; c++) tot[c] += sh.tsum[c][w];
-        if (!all) {
+        if (!all && sh.ok) {                       // not the sums of a poll that ran out
           if (xi == 0u)
             for (int k = lane; k < kTeamSums * M.T; k += 32)
               sums_put<NP>(tp, xi, 1, M.slot0 + k / kTeamSums, tot, ep, k % kTeamSums);

@@ -137,6 +137,28 @@ def test_more_basins_than_a_grid_has_rows():
         assert a.info(0).volume == m.info(i).volume > 0
 
 
+@pytest.mark.parametrize("nx,ny,opts", [(41, 25, {}), (514, 514, {}), (41, 25, dict(zeta_tile_rows=512)),
+                                        (41, 25, dict(zeta_stage=1))])
+def test_bounded_waits(nx, ny, opts):
+    """A wait for a member (resident: two, and 130, which send their sums
+    through member 0) or an arrival (streaming) that does not exist runs out,
+    the step reports it, and the same model then runs as if it had not been."""
+    c = cases.channel_case(nx=nx, ny=ny, lx=150.0 * (nx - 1), ly=150.0 * (ny - 1))
+    ref, m = run(c, 1, **opts), shygpu.Model(c)
+    for k, v in opts.items():
+        m.set_option(k, v)
+    m.set_state(0)
+    m.set_option("zeta_barrier_timeout_test", 1)
+    with pytest.raises(shygpu.ShyError) as e:
+        m.run(1)
+    assert e.value.code == 2 and "ran out" in str(e.value)
+    m.set_option("zeta_barrier_timeout_test", 0)
+    for g in (ref, m):                                       # both clocks have made one step
+        g.set_state(0)
+        g.run(3)
+    assert np.array_equal(znv(m), znv(ref))
+
+
 def test_levels_across_the_wrap_of_the_launch_number():
     """The resident solver numbers its launches with 16 bits: twelve steps
     across the wrap give the levels that the cluster solver gives."""
