@@ -647,7 +647,7 @@ def main():
     prof = model.profile_steps(20)
     infos = [model.info(b) for b in range(nb)]
     nsc = int(c0["params"]["itemp"]) + int(c0["params"]["isalt"]) + int(c0["params"]["nconz"])
-    resident = model.get_option("zeta_variant") == 2 and model.get_option("zeta_stage") == 0
+    resident = model.get_option("zeta_resident") == 1
     algo = algorithmic_bytes(case_list, infos, nsc, resident=resident)
     tot_ms = sum(v[0] for v in prof.values())
     dom = max(prof, key=lambda k: prof[k][0])
@@ -682,7 +682,7 @@ def main():
                 "per_basin": {"value": pb_value, "steps": pb_steps,
                               "path": "shygpu_set_forcing(wind) + shygpu_run(1) + shygpu_get_state(znv), "
                                       "every basin, waiting after each call"}},
-        "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak,
+        "roofline": {"bound": "latency" if dom == "zeta" and resident else "hbm", "kernel": dom, "achieved": achieved, "peak": peak,
                      "peak_source": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "algorithmic_bytes_per_launch": dom_bytes,
                      "bytes_model": ("zeta: 100 B per node for assembly + 80 B per node per CG "

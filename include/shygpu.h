@@ -387,7 +387,9 @@ int shygpu_set_bound_scalar(shygpu_model *model, int32_t ibasin, int32_t what,
  * another value selects it),
  * "zeta_barrier_timeout_test" (failure detection: the device-wide solve's
  * barrier waits for an arrival that never comes and reports SHY_ECUDA).
- * Every change rebuilds the step graphs at the next step.                  */
+ * Every change rebuilds the step graphs at the next step.  To read only:
+ * "zeta_resident" and "nh_resident" (1 where the zeta systems, the 3D
+ * pressure systems, are on the resident solver).                          */
 int shygpu_set_option(shygpu_model *model, const char *name, double value);
 double shygpu_get_option(shygpu_model *model, const char *name);
 

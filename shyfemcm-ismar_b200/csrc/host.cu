@@ -1523,6 +1523,8 @@ extern "C" double shygpu_get_option(shygpu_model *m, const char *name) {
   if (n == "max_outer") return m->max_outer;
   if (n == "symmetric") return m->sym;
   if (n == "zeta_variant") return m->zcl.empty() ? -1 : (m->zcl[0].grid || m->zcl[0].team ? 2 : 0);
+  if (n == "zeta_resident") return m->zcl.empty() ? -1 : m->zcl[0].team;
+  if (n == "nh_resident") return m->nh_TG > 0;
   if (n == "zeta_grid_ctas") return m->zcl.empty() ? -1 : m->zcl[0].G;
   if (n == "zeta_stage") return m->zcl.empty() || !m->zcl[0].grid ? m->zstage : (m->zcl[0].staged ? 1 : 0);
   if (n == "zeta_tile_rows") return m->ztile_rows > 0 ? m->ztile_rows : zeta_grid_tile_rows();

@@ -172,3 +172,24 @@ def test_levels_across_the_wrap_of_the_launch_number():
     m.set_option("zeta_variant", 0)
     m.run(12)
     assert np.abs(a).max() > 0.01 and np.abs(a - znv(m)).max() <= 1.0e-5
+
+
+def solvers(m):
+    return m.get_option("zeta_variant"), m.get_option("zeta_resident"), m.get_option("nh_resident")
+
+
+def test_which_solver_runs():
+    """The plan each option selects, as get_option tells it."""
+    c = cases.channel_case()
+    assert solvers(shygpu.Model(c)) == (2, 1, 0)
+    rotating = dict(c, fcorv=np.full(c["nel"], 1.0e-4, np.float32))
+    for case, opts, want in ((c, dict(zeta_variant=2), (2, 1)), (c, dict(zeta_variant=0), (0, 0)),
+                             (c, dict(zeta_tile_rows=512), (2, 0)), (c, dict(zeta_tile_rows=1024), (2, 1)),
+                             (c, dict(zeta_stage=1), (2, 0)), (c, dict(symmetric=0), (2, 1)),
+                             (rotating, {}, (2, 1)), (rotating, dict(zeta_tile_rows=512), (2, 1)),
+                             (rotating, dict(zeta_variant=0), (0, 0))):
+        m = shygpu.Model(case)
+        for k, v in opts.items():
+            m.set_option(k, v)
+        assert solvers(m)[:2] == want, opts
+    assert solvers(shygpu.Model(cases.seiche_case())) == (2, 1, 1)
