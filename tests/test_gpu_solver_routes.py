@@ -193,3 +193,50 @@ def test_which_solver_runs():
             m.set_option(k, v)
         assert solvers(m)[:2] == want, opts
     assert solvers(shygpu.Model(cases.seiche_case())) == (2, 1, 1)
+
+
+def parity(c, g, o):
+    a, b = g.get_state(0), o.state()
+    assert np.abs(a["znv"] - b["znv"]).max() <= ZETA_TOL
+    act = np.arange(c["nlv"])[None, :] < c["ilhkv"][:, None]
+    for f in ("tempv", "saltv"):
+        assert np.abs(a[f] - b[f])[act].max() <= 1.0e-4 * np.abs(b[f][act]).max(), f
+
+
+@pytest.mark.parametrize("tile_rows", [128, 512, 2048])
+def test_streaming_solver_matches_the_oracle(small3d, tile_rows):
+    """The streaming solver with plain loads on the 3D basin (tracers to the
+    parity tolerance, 1e-4)."""
+    g = run(small3d, 120, zeta_tile_rows=tile_rows)
+    assert solvers(g)[:2] == (2, 0) and g.get_option("zeta_stage") == 0
+    o = shyref.OracleModel(small3d)
+    o.run(120)
+    parity(small3d, g, o)
+    assert g.info(0).krylov_iters > 0
+
+
+def test_streaming_solver_in_a_mix():
+    """Basins of very different sizes on the streaming solver: the bits that
+    each has alone on it, and the resident solver's levels."""
+    cs = [cases.basin3d_case(nkn_target=n, nlv=4, seed=s, baroclinic=False, ts=False)
+          for n, s in ((50000, 21), (700, 22), (3000, 23))]
+    gb = run(cs, 20, zeta_tile_rows=512)
+    assert solvers(gb)[:2] == (2, 0)
+    for i, c in enumerate(cs):
+        assert np.array_equal(znv(run(c, 20, zeta_tile_rows=512)), znv(gb, i)), i
+        r = run(c, 20)
+        assert solvers(r)[:2] == (2, 1)
+        assert np.abs(znv(r) - znv(gb, i)).max() <= 1.0e-5, i
+
+
+def test_full_ensemble_on_the_streaming_solver():
+    """The 64-basin ensemble at its full size: members have the bits that
+    they have alone, and the resident solver's levels."""
+    ens = cases.ensemble_cases(64)
+    g, r = run(ens, 6, zeta_tile_rows=512), run(ens, 6)
+    assert solvers(g)[:2] == (2, 0) and solvers(r)[:2] == (2, 1)
+    sizes = [c["nkn"] for c in ens]
+    for i in (int(np.argmax(sizes)), int(np.argmin(sizes)), 17):
+        assert np.array_equal(znv(run(ens[i], 6, zeta_tile_rows=512)), znv(g, i)), i
+    for i in range(len(ens)):
+        assert np.abs(znv(g, i) - znv(r, i)).max() <= 1.0e-5, i
