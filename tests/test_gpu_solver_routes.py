@@ -240,3 +240,55 @@ def test_full_ensemble_on_the_streaming_solver():
         assert np.array_equal(znv(run(ens[i], 6, zeta_tile_rows=512)), znv(g, i)), i
     for i in range(len(ens)):
         assert np.abs(znv(g, i) - znv(r, i)).max() <= 1.0e-5, i
+
+
+@pytest.mark.parametrize("coriolis", [0.0, 1.0e-4])
+def test_basin_too_wide_for_the_resident_solver(coriolis):
+    """313600 rows need more CTAs than the device has resident: the whole
+    batch goes to the streaming solver (symmetric) or the clusters."""
+    cs = [cases.channel_case(nx=n, ny=n, lx=150.0 * (n - 1), ly=150.0 * (n - 1)) for n in (560, 24)]
+    for c in cs:
+        c["fcorv"] = np.full(c["nel"], coriolis, np.float32)
+    g, ref = run(cs, 3), run(cs, 3, zeta_variant=0)
+    assert solvers(g)[:2] == ((2, 0) if coriolis == 0.0 else (0, 0))
+    small = run(cs[1], 3)
+    assert solvers(small)[:2] == (2, 1)
+    assert np.abs(znv(small) - znv(g, 1)).max() <= 1.0e-5
+    for i in range(2):
+        assert np.abs(znv(g, i) - znv(ref, i)).max() <= 1.0e-5, i
+
+
+@pytest.mark.parametrize("coriolis", [0.0, 1.0e-4])
+def test_share_with_too_many_ghosts(coriolis):
+    """A hub of 1400 neighbours: its share would hold more ghosts than a CTA
+    has places, so the model runs another solver, and so does a basin beside
+    it that would fit."""
+    c, other = disc(1400, rings=3, r0=1000.0), cases.channel_case()
+    for q in (c, other):
+        q["fcorv"] = np.full(q["nel"], coriolis, np.float32)
+    g = run([c, other], 5)
+    assert solvers(g)[:2] == ((2, 0) if coriolis == 0.0 else (0, 0))
+    o = shyref.OracleModel(c)
+    o.run(5)
+    assert np.abs(znv(g) - o.state()["znv"]).max() <= ZETA_TOL
+    assert np.abs(znv(run(other, 5)) - znv(g, 1)).max() <= 1.0e-5
+
+
+@pytest.mark.parametrize("what", ["hub", "rows"])
+def test_pressure_system_that_does_not_fit(what):
+    """A share with too many ghosts (a hub of 800 neighbours), or more rows
+    (84252) than are resident: the pressure goes to its own device-wide
+    solver, for a basin beside it as well."""
+    c = nh_disc(800) if what == "hub" else cases.nh_basin_case(nkn_target=7000, lx=600.0, ly=300.0, nlv=12)
+    other = cases.seiche_case()
+    g, o, alone = run([c, other], 3), shyref.OracleModel(c), run(other, 3)
+    o.run(3)
+    assert solvers(g)[2] == 0 and solvers(alone)[2] == 1
+    z, (q, (it, _, r0, r)), qo = o.state()["znv"], g.nh(0), o.nh()[0]
+    assert np.abs(znv(g) - z).max() <= 1.0e-3 * max(np.abs(z).max(), 1.0e-3)
+    assert it > 0 and r <= 1e-8 * r0 + 1e-8
+    act = np.arange(c["nlv"])[None, :] < c["ilhkv"][:, None]
+    assert np.abs(q - qo)[act].max() <= 1.0e-2 * np.abs(qo[act]).max()
+    qa, qb = alone.nh(0)[0], g.nh(1)[0]
+    assert np.abs(qa - qb).max() <= 1.0e-2 * np.abs(qa).max()
+    assert np.abs(znv(alone) - znv(g, 1)).max() <= 1.0e-5
