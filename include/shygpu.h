@@ -372,8 +372,9 @@ int shygpu_set_bound_scalar(shygpu_model *model, int32_t ibasin, int32_t what,
 
 /* Tuning options by name: "use_graph" (CUDA-graph replay of whole steps,
  * the transport sub-step loop as a device-driven conditional node; default
- * 1), "cluster_size" and "zeta_threads" (shape of the per-basin cluster of
- * the zeta solve), "zeta_variant" (0 cluster solver with vectors in global
+ * 1), "cluster_size" and "zeta_threads" (shape of the per-basin clusters
+ * where they solve zeta: zeta_variant 0, or a basin that fits no other
+ * solver), "zeta_variant" (0 cluster solver with vectors in global
  * memory; 1, 2 one device-wide cooperative solve: the resident solver, or
  * the streaming one when a basin does not fit it), "zeta_stage" (streaming
  * solve with TMA-staged tiles), "inner_rtol" (residual reduction of each

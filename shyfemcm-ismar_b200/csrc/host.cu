@@ -720,8 +720,13 @@ static int build_team_class(shygpu_model *m) {
 
 static int build_zeta_plan_impl(shygpu_model *m, int forceCL, int forceThreads);
 
-// forceCL > 0: one class with that shape for every basin.  A plan that
-// cannot be built leaves no plan (the step then refuses to run).
+// the clusters of a basin of nk rows where no shape is asked for
+static const int kClusterThreads = 1024;
+static int cluster_size_of(int nk) { return std::min(16, next_pow2((nk + 4095) / 4096)); }
+
+// forceCL > 0: where clusters solve, one class with that shape for every
+// basin.  A plan that cannot be built leaves no plan (the step then refuses
+// to run).
 static int build_zeta_plan(shygpu_model *m, int forceCL, int forceThreads) {
   int st = build_zeta_plan_impl(m, forceCL, forceThreads);
   if (st == SHY_OK) st = settle();
@@ -734,7 +739,8 @@ static int build_zeta_plan_impl(shygpu_model *m, int forceCL, int forceThreads) 
   // zeta_variant 1 and 2: the resident solver where every basin fits it, else,
   // or when its tiles are asked for, the streaming device-wide solver for
   // symmetric systems
-  if (m->zvariant && forceCL <= 0) {
+  if (forceCL > 0) ST_TRY(check_cluster_shape(forceCL, forceThreads));
+  if (m->zvariant) {
     int st = SHY_EARG;
     if (!m->sym || (!m->zstage && (m->ztile_rows == 0 || m->ztile_rows == zeta_grid_tile_rows()))) st = build_team_class(m);
     if (st == SHY_EARG && m->sym) {
@@ -754,8 +760,8 @@ static int build_zeta_plan_impl(shygpu_model *m, int forceCL, int forceThreads) 
   // any batch
   int maxCL = 1;
   for (int b = 0; b < m->nbasin; b++) {
-    const int CL = forceCL > 0 ? forceCL : std::min(16, next_pow2((m->par[b].nk + 4095) / 4096));
-    const int th = forceCL > 0 ? forceThreads : 1024;
+    const int CL = forceCL > 0 ? forceCL : cluster_size_of(m->par[b].nk);
+    const int th = forceCL > 0 ? forceThreads : kClusterThreads;
     ZetaClass *cls = nullptr;
     for (ZetaClass &c : m->zcl)
       if (c.CL == CL) cls = &c;
@@ -1432,9 +1438,12 @@ extern "C" int shygpu_set_option(shygpu_model *m, const char *name, double value
   int iv = (int)value;
   if (n == "use_graph") m->use_graph = iv != 0;
   else if (n == "cluster_size" || n == "zeta_threads") {
-    // one launch class with this shape for every basin (0 returns to the automatic plan)
-    int CL = m->zforce_CL > 0 ? m->zforce_CL : (m->zcl.empty() ? 1 : m->zcl[0].CL);
-    int th = m->zforce_threads > 0 ? m->zforce_threads : (m->zcl.empty() ? 512 : m->zcl[0].threads);
+    // one launch class with this shape for every basin where clusters solve
+    // (0 returns to the automatic plan); the device-wide solvers keep their
+    // own shapes, and are faster (7000 rows: 175 us a step, clusters of 1 to
+    // 16 with vectors in shared memory, which they replaced, 5000 to 248 us)
+    int CL = m->zforce_CL > 0 ? m->zforce_CL : cluster_size_of(m->par[0].nk);
+    int th = m->zforce_threads > 0 ? m->zforce_threads : kClusterThreads;
     if (n == "cluster_size") {
       if (iv != 0 && (iv < 1 || iv > 16 || (iv & (iv - 1)))) return fail(SHY_EARG, "cluster_size: power of two 1..16");
       CL = iv;
@@ -1512,8 +1521,8 @@ extern "C" double shygpu_get_option(shygpu_model *m, const char *name) {
   if (!m || !name) return -1;
   std::string n(name);
   if (n == "use_graph") return m->use_graph;
-  if (n == "cluster_size") return m->zcl.empty() ? -1 : m->zcl[0].CL;
-  if (n == "zeta_threads") return m->zcl.empty() ? -1 : m->zcl[0].threads;
+  if (n == "cluster_size") return m->zcl.empty() ? -1 : (m->zforce_CL > 0 ? m->zforce_CL : m->zcl[0].CL);
+  if (n == "zeta_threads") return m->zcl.empty() ? -1 : (m->zforce_threads > 0 ? m->zforce_threads : m->zcl[0].threads);
   if (n == "zeta_classes") return (double)m->zcl.size();
   if (n == "column_threads") return m->base.col_threads;
   if (n == "column_staged") return m->base.col_staged;

@@ -292,3 +292,30 @@ def test_pressure_system_that_does_not_fit(what):
     qa, qb = alone.nh(0)[0], g.nh(1)[0]
     assert np.abs(qa - qb).max() <= 1.0e-2 * np.abs(qa).max()
     assert np.abs(znv(alone) - znv(g, 1)).max() <= 1.0e-5
+
+
+def test_cluster_shape():
+    """cluster_size and zeta_threads are kept and told back whatever solver
+    runs, hold where clusters solve, and a shape that cannot be is refused."""
+    c = cases.channel_case(nx=41, ny=25)
+    m = shygpu.Model(c)
+    m.set_option("cluster_size", 4)
+    shape = lambda m: (m.get_option("cluster_size"), m.get_option("zeta_threads"))
+    assert shape(m) == (4, 1024) and solvers(m)[:2] == (2, 1)
+    m.set_option("zeta_threads", 256)
+    assert shape(m) == (4, 256) and solvers(m)[:2] == (2, 1)
+    m.set_state(0)
+    m.run(3)
+    assert np.array_equal(znv(m), znv(run(c, 3)))
+    m.set_option("zeta_variant", 0)
+    assert shape(m) == (4, 256) and solvers(m)[:2] == (0, 0)
+    a = run(c, 3, zeta_variant=0, zeta_threads=256, cluster_size=4)
+    b = run(c, 3, cluster_size=4, zeta_threads=256, zeta_variant=0)
+    assert np.array_equal(znv(a), znv(b)) and np.abs(znv(a) - znv(run(c, 3))).max() <= 1.0e-5
+    for name, value in (("cluster_size", 3), ("cluster_size", 32), ("zeta_threads", 100), ("zeta_threads", 2048)):
+        with pytest.raises(shygpu.ShyError):
+            m.set_option(name, value)
+    m.set_option("cluster_size", 0)
+    assert shape(m) == (1, 1024)
+    m.set_option("zeta_variant", 1)
+    assert solvers(m)[:2] == (2, 1)
