@@ -328,6 +328,7 @@ struct shygpu_model {
   cudaStream_t xin = nullptr, xout = nullptr;
   float *fstage[2][4] = {};
   size_t fstage_bytes = 0;
+  int64_t plan_bytes = 0;            // of the zeta plan on the device
   cudaEvent_t ev_fin[2] = {}, ev_fused[2] = {}, ev_done = nullptr, ev_lev[2] = {};
   bool fused_rec[2] = {false, false}, lev_pending[2] = {false, false};
   int fgen = 0;
@@ -404,6 +405,7 @@ static void free_zeta_plan(shygpu_model *m) {
     }
   }
   m->zcl.clear();
+  m->plan_bytes = 0;
 }
 
 // The device-wide class: every basin in one cooperative launch.  Each
@@ -414,8 +416,15 @@ static void free_zeta_plan(shygpu_model *m) {
 // iterate is shared out.  Returns SHY_EARG when a CTA would hold more tiles
 // or basins than it can.
 template <typename T>
-static int upload_plan(T **dst, const std::vector<T> &h) {
-  CUDA_TRY(cudaMalloc((void **)dst, sizeof(T) * std::max<size_t>(h.size(), 1)));
+static int plan_alloc(shygpu_model *m, T **dst, size_t n) {
+  CUDA_TRY(cudaMalloc((void **)dst, sizeof(T) * std::max<size_t>(n, 1)));
+  m->plan_bytes += (int64_t)(sizeof(T) * std::max<size_t>(n, 1));
+  return SHY_OK;
+}
+
+template <typename T>
+static int upload_plan(shygpu_model *m, T **dst, const std::vector<T> &h) {
+  ST_TRY(plan_alloc(m, dst, h.size()));
   if (!h.empty()) CUDA_TRY(cudaMemcpy(*dst, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
   return SHY_OK;
 }
@@ -519,49 +528,49 @@ static int build_grid_class(shygpu_model *m) {
   c.gp.phantom = m->zbar_test ? 1u : 0u;
   c.gp.spin_limit = m->zbar_test ? (1LL << 14) : zeta_grid_spin_limit();
   int4 *dt = nullptr; int2 *dbt = nullptr; int *dcs = nullptr, *dcn = nullptr, *dco = nullptr;
-  ST_TRY(upload_plan(&dt, tile)); c.gp.tile = dt;
-  ST_TRY(upload_plan(&dbt, btile)); c.gp.btile = dbt;
-  ST_TRY(upload_plan(&dcs, cslot)); c.gp.cslot = dcs;
-  ST_TRY(upload_plan(&dcn, cnslot)); c.gp.cnslot = dcn;
-  ST_TRY(upload_plan(&dco, cowner)); c.gp.cowner = dco;
+  ST_TRY(upload_plan(m, &dt, tile)); c.gp.tile = dt;
+  ST_TRY(upload_plan(m, &dbt, btile)); c.gp.btile = dbt;
+  ST_TRY(upload_plan(m, &dcs, cslot)); c.gp.cslot = dcs;
+  ST_TRY(upload_plan(m, &dcn, cnslot)); c.gp.cnslot = dcn;
+  ST_TRY(upload_plan(m, &dco, cowner)); c.gp.cowner = dco;
   int *dcp = nullptr, *dcl = nullptr;
-  ST_TRY(upload_plan(&dcp, cptr)); c.gp.cptr = dcp;
-  ST_TRY(upload_plan(&dcl, clist)); c.gp.clist = dcl;
+  ST_TRY(upload_plan(m, &dcp, cptr)); c.gp.cptr = dcp;
+  ST_TRY(upload_plan(m, &dcl, clist)); c.gp.clist = dcl;
   // the scaled system's arrays; the corrections carry 16 bytes of slack that
   // the staged form's widened copies may touch
   {
     int *des = nullptr;
-    ST_TRY(upload_plan(&des, eslot)); c.gp.eslot = des;
+    ST_TRY(upload_plan(m, &des, eslot)); c.gp.eslot = des;
     if (c16) {
       std::vector<short> oc((size_t)EW * NKN);
       for (int i = 0; i < NKN; i++)
         for (int k = 0; k < EW; k++) oc[(size_t)EW * i + k] = (short)(ecol[(size_t)EW * i + k] - i);
       short *d16 = nullptr;
-      ST_TRY(upload_plan(&d16, oc)); c.gp.ecol16 = d16;
+      ST_TRY(upload_plan(m, &d16, oc)); c.gp.ecol16 = d16;
     } else {
       int *d32 = nullptr;
-      ST_TRY(upload_plan(&d32, ecol)); c.gp.ecol32 = d32;
+      ST_TRY(upload_plan(m, &d32, ecol)); c.gp.ecol32 = d32;
     }
-    CUDA_TRY(cudaMalloc(&c.gp.eval, sizeof(float) * EW * (size_t)NKN));
+    ST_TRY(plan_alloc(m, &c.gp.eval, EW * (size_t)NKN));
     CUDA_TRY(cudaMemset(c.gp.eval, 0, sizeof(float) * EW * (size_t)NKN));
     c.gp.nx = (int)nx;
     if (nx) {
       int *dxp = nullptr, *dxc = nullptr, *dxs = nullptr;
-      ST_TRY(upload_plan(&dxp, xptr)); c.gp.xptr = dxp;
-      ST_TRY(upload_plan(&dxc, xcol)); c.gp.xcol = dxc;
-      ST_TRY(upload_plan(&dxs, xslot)); c.gp.xslot = dxs;
-      CUDA_TRY(cudaMalloc(&c.gp.xval, sizeof(float) * nx));
+      ST_TRY(upload_plan(m, &dxp, xptr)); c.gp.xptr = dxp;
+      ST_TRY(upload_plan(m, &dxc, xcol)); c.gp.xcol = dxc;
+      ST_TRY(upload_plan(m, &dxs, xslot)); c.gp.xslot = dxs;
+      ST_TRY(plan_alloc(m, &c.gp.xval, nx));
     }
-    CUDA_TRY(cudaMalloc(&c.gp.sd, sizeof(float) * (NKN + 8)));
-    CUDA_TRY(cudaMalloc(&c.gp.ecor, sizeof(float) * (NKN + 8)));
+    ST_TRY(plan_alloc(m, &c.gp.sd, (size_t)NKN + 8));
+    ST_TRY(plan_alloc(m, &c.gp.ecor, (size_t)NKN + 8));
     CUDA_TRY(cudaMemset(c.gp.ecor, 0, sizeof(float) * (NKN + 8)));
   }
   for (float4 *&p : c.gp.cg4) {
-    CUDA_TRY(cudaMalloc(&p, sizeof(float4) * NKN));
+    ST_TRY(plan_alloc(m, &p, NKN));
     CUDA_TRY(cudaMemset(p, 0, sizeof(float4) * NKN));
   }
-  CUDA_TRY(cudaMalloc(&c.gp.partial, sizeof(double) * 8 * std::max<size_t>(tile.size(), 1)));
-  CUDA_TRY(cudaMalloc(&c.gp.ctr, 8 * sizeof(unsigned)));
+  ST_TRY(plan_alloc(m, &c.gp.partial, 8 * std::max<size_t>(tile.size(), 1)));
+  ST_TRY(plan_alloc(m, &c.gp.ctr, 8));
   CUDA_TRY(cudaMemset(c.gp.ctr, 0, 8 * sizeof(unsigned)));
   return SHY_OK;
 }
@@ -680,6 +689,7 @@ static int make_team_plan(TeamPlan &t, int &G, const TeamShape &sh, const std::v
   char *base = nullptr;
   CUDA_TRY(cudaMalloc(&base, bytes));
   t.base = base;
+  t.bytes = (int64_t)bytes;
   CUDA_TRY(cudaMemcpy(base, image.data(), image.size(), cudaMemcpyHostToDevice));
   CUDA_TRY(cudaMemset(base + copied, 0, bytes - copied));
   t.mem = (const TeamMember *)(base + o_mem);
@@ -715,7 +725,9 @@ static int build_team_class(shygpu_model *m) {
   c.team = true;
   c.CL = c.threads = 0;
   for (int i = 0; i < m->nbasin; i++) c.basins.push_back(i);
-  return make_team_plan(c.tp, c.G, zeta_team_shape(), m->rowptr_h, m->col_h, m->xy_h, jobs, m->zbar_test != 0);
+  ST_TRY(make_team_plan(c.tp, c.G, zeta_team_shape(), m->rowptr_h, m->col_h, m->xy_h, jobs, m->zbar_test != 0));
+  m->plan_bytes += c.tp.bytes;
+  return SHY_OK;
 }
 
 static int build_zeta_plan_impl(shygpu_model *m, int forceCL, int forceThreads);
@@ -780,7 +792,7 @@ static int build_zeta_plan_impl(shygpu_model *m, int forceCL, int forceThreads) 
     if (e != cudaSuccess) return fail(SHY_ECUDA, "zeta kernel setup: %s", cudaGetErrorString(e));
   }
   for (ZetaClass &c : m->zcl) {
-    CUDA_TRY(cudaMalloc(&c.d_blist, sizeof(int) * c.basins.size()));
+    ST_TRY(plan_alloc(m, &c.d_blist, c.basins.size()));
     CUDA_TRY(cudaMemcpy(c.d_blist, c.basins.data(), sizeof(int) * c.basins.size(), cudaMemcpyHostToDevice));
   }
   if ((int)m->zcl.size() > kMaxZetaClasses) return fail(SHY_EARG, "too many zeta launch classes");
@@ -855,7 +867,7 @@ extern "C" int64_t shygpu_footprint(int32_t nbasin, const shy_basin *basins, con
 }
 
 extern "C" int64_t shygpu_model_bytes(const shygpu_model *m) {
-  return m ? (int64_t)(m->arena.held + m->fstage_bytes) : -1;
+  return m ? (int64_t)(m->arena.held + m->fstage_bytes + m->plan_bytes + m->nh_team.bytes) : -1;
 }
 
 // the streams and events of the pipelined transfers, made on first use

@@ -137,6 +137,7 @@ struct TeamPlan {
   // the system of the CSR instance: FP64 matrix and right-hand side, solution
   struct { const int *rowptr; const double *val, *rhs; float *x; } csr = {nullptr, nullptr, nullptr, nullptr};
   void *base = nullptr;            // the allocation that holds the arrays below
+  int64_t bytes = 0;               // its size
   const TeamMember *mem = nullptr;
   const int *cptr = nullptr, *clist = nullptr;
   const int *rows = nullptr, *dpos = nullptr, *ghost = nullptr;

@@ -319,3 +319,21 @@ def test_cluster_shape():
     assert shape(m) == (1, 1024)
     m.set_option("zeta_variant", 1)
     assert solvers(m)[:2] == (2, 1)
+
+
+def test_model_bytes_count_the_plan():
+    """What shygpu_model_bytes adds for each zeta plan: per row 4 + 4 + 16
+    (row, lengths, columns) + 32 (exchange words) bytes resident, 32 + 16 +
+    32 + 8 + 32 streaming, and a little more for ghosts, sums and lists."""
+    c = cases.channel_case(nx=200, ny=150, lx=150.0 * 199, ly=150.0 * 149)
+    n = c["nkn"]
+    size = {}
+    m = shygpu.Model(c)
+    for name, opts in (("resident", {}), ("streaming", dict(zeta_tile_rows=512)), ("clusters", dict(zeta_variant=0)),
+                       ("again", dict(zeta_tile_rows=0, zeta_variant=1))):
+        for k, v in opts.items():
+            m.set_option(k, v)
+        size[name] = m.nbytes()
+    assert 56 * n <= size["resident"] - size["clusters"] <= 64 * n
+    assert 120 * n <= size["streaming"] - size["clusters"] <= 128 * n
+    assert size["again"] == size["resident"]
