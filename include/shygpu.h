@@ -404,7 +404,8 @@ double shygpu_get_option(shygpu_model *model, const char *name);
  * steps; the search takes one group at a time over the best of the groups
  * before it.  The model keeps the fastest candidate's options and the state
  * it had.  The winner is cached per model shape (basins, rows to two
- * digits, layers, solver, scalars, device) for the process, and appended to
+ * digits, layers, solver, scalars, device) and meaning of the options (a
+ * choice kept from before they selected other kernels is not applied) for the process, and appended to
  * the file named by the environment variable SHYGPU_TUNE_FILE, if set, which
  * later processes read; a cached shape is applied without trials.  choice
  * (optional) receives the options as "name=value ...", ms_per_step

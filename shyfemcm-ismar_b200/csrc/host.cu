@@ -2751,18 +2751,25 @@ std::mutex g_tune_mu;
 std::map<std::string, std::string> g_tune_cache;
 bool g_tune_file_read = false;
 
+// Raised when an option of the candidates comes to select another kernel, so
+// that choices kept from before are measured again: 2 since zeta_variant 1
+// and 2 select the resident solver (an ensemble tuned before that, to tiles
+// of the streaming solver, would stay on it: 5.05 against 2.71 ms a solve).
+constexpr int kTunePlans = 2;
+
 std::string tune_key(const shygpu_model *m) {
-  // what decides the winner: basins, total rows to two digits, layers, the
-  // solver's symmetry, Coriolis, wetting and drying, transported scalars,
-  // and the device
+  // what decides the winner: the candidates and what their options select
+  // (kTunePlans), basins, total rows to two digits, layers, the solver's
+  // symmetry, Coriolis, wetting and drying, transported scalars, and the
+  // device
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   long long rows = m->NKN, scale = 1;
   while (rows >= 100) { rows /= 10; scale *= 10; }
   char k[256];
-  snprintf(k, sizeof k, "nbasin=%d rows=%lld nlv=%d sym=%d cor=%d wd=%d nsc=%d sm=%d", m->nbasin, rows * scale,
-           m->NLV, (int)m->sym, (int)m->cor, (int)m->any_wd, m->nsc_max, nsm);
+  snprintf(k, sizeof k, "plans=%d nbasin=%d rows=%lld nlv=%d sym=%d cor=%d wd=%d nsc=%d sm=%d", kTunePlans, m->nbasin,
+           rows * scale, m->NLV, (int)m->sym, (int)m->cor, (int)m->any_wd, m->nsc_max, nsm);
   return k;
 }
 

@@ -337,3 +337,25 @@ def test_model_bytes_count_the_plan():
     assert 56 * n <= size["resident"] - size["clusters"] <= 64 * n
     assert 120 * n <= size["streaming"] - size["clusters"] <= 128 * n
     assert size["again"] == size["resident"]
+
+
+def test_tuned_choices_of_other_plans_are_measured_again(tmp_path):
+    """A tune file whose entry names no plans (the options selected other
+    solvers then) is not applied; the entry that replaces it is."""
+    import os
+    import subprocess
+    import sys
+    import torch
+
+    sm = torch.cuda.get_device_properties(0).multi_processor_count
+    f = tmp_path / "tune"
+    f.write_text(f"nbasin=1 rows=790 nlv=1 sym=1 cor=0 wd=0 nsc=0 sm={sm}\t"
+                 "zeta_stage=0 zeta_tile_rows=512 zeta_variant=2 inner_tol_frac=0.75\n")
+    code = ("import shygpu; from shygpu import cases\n"
+            "m = shygpu.Model(cases.channel_case()); m.set_state(0)\n"
+            "print(m.autotune(steps=2)[1] == -1.0)")
+    env = dict(os.environ, SHYGPU_TUNE_FILE=str(f), PYTHONPATH=os.pathsep.join(sys.path))
+    out = [subprocess.run([sys.executable, "-c", code], env=env, check=True, capture_output=True,
+                          text=True).stdout.split()[-1] for _ in range(2)]
+    assert out == ["False", "True"]
+    assert len(f.read_text().splitlines()) == 2
