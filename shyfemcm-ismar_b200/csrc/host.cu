@@ -599,18 +599,11 @@ static int make_team_plan(TeamPlan &t, int &G, const TeamShape &sh, const std::v
   }
   // the systems' shares, on the host's cores
   std::vector<TeamBasin> tb(NB);
-  {
-    std::atomic<int> next{0};
-    auto work = [&] {
-      for (int b; (b = next++) < NB;)
+  const int nt = nrows < 100000 ? 1 : std::min(8, (int)std::thread::hardware_concurrency());
+  if (!on_threads(NB, nt, [&](int b) {
         team_basin(rowptr.data(), col.data(), xy.data(), jobs[b].k0, jobs[b].nk, jobs[b].width, sh, tb[b]);
-    };
-    const int nt = nrows < 100000 ? 1 : std::min(NB, std::max(1, std::min(8, (int)std::thread::hardware_concurrency())));
-    std::vector<std::thread> pool;
-    for (int q = 1; q < nt; q++) pool.emplace_back(work);
-    work();
-    for (std::thread &q : pool) q.join();
-  }
+      }))
+    return fail(SHY_ECAPACITY, "resident solver: no host memory for the plan");
   std::vector<TeamMember> mem;
   std::vector<int> first(NB + 1, 0), ord, dpos, ghost, tptr(1, 0), tslot;
   std::vector<unsigned short> lcol, tcol;

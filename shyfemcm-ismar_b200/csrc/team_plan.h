@@ -5,7 +5,9 @@
 // a plain C++ compiler.
 #pragma once
 #include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <thread>
 #include <vector>
 
 #ifdef __CUDACC__
@@ -31,6 +33,29 @@ struct TeamShape {
 SHY_HD int dpos_pack(int place, int count) { return place | count << 16; }
 SHY_HD int dpos_place(int v) { return v & 0xffff; }
 SHY_HD int dpos_count(int v) { return (int)((unsigned)v >> 16); }
+
+// fn(i) for i = 0 .. n-1 on up to nt threads, the caller's among them; false
+// when a call threw.  Threads that the system refuses are done without.
+template <class F>
+inline bool on_threads(int n, int nt, F fn) {
+  std::atomic<int> next{0};
+  std::atomic<bool> ok{true};
+  auto work = [&] {
+    try {
+      for (int i; (i = next++) < n;) fn(i);
+    } catch (...) {
+      ok = false;
+    }
+  };
+  std::vector<std::thread> pool;
+  try {
+    for (int q = 1; q < std::min(n, nt); q++) pool.emplace_back(work);
+  } catch (...) {
+  }
+  work();
+  for (std::thread &t : pool) t.join();
+  return ok;
+}
 
 // a row with its place in the plane
 struct PlaneRow { float x[2]; int i; };

@@ -35,17 +35,32 @@ extern "C" int deal(int nk, const int *rowptr, const int *col, const float *xy, 
     }
   return n;
 }
+// n pieces of work on nt threads, the one numbered `bad` throwing: how many
+// were done, negative when on_threads says that one threw
+extern "C" int pieces(int n, int nt, int bad) {
+  std::atomic<int> done{0};
+  const bool ok = on_threads(n, nt, [&](int i) {
+    if (i == bad) throw std::bad_alloc();
+    done++;
+  });
+  return ok ? (int)done : -(int)done;
+}
 """
 
 
 @pytest.fixture(scope="module")
-def deal(tmp_path_factory):
+def lib(tmp_path_factory):
     d = tmp_path_factory.mktemp("plan")
     (d / "plan.cpp").write_text(HARNESS)
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-pthread", f"-I{CSRC}", str(d / "plan.cpp"), "-o",
                     str(d / "plan.so")], check=True)
     lib = C.CDLL(str(d / "plan.so"))
+    lib.path = str(d / "plan.so")
+    return lib
 
+
+@pytest.fixture(scope="module")
+def deal(lib):
     def call(pattern, xy, T, rows=2048, ghosts=512, entries=8):
         nk = len(pattern)
         rowptr = np.r_[0, np.cumsum([len(p) for p in pattern])].astype(np.int32)
@@ -109,3 +124,26 @@ def test_shares_of_a_hub(deal, T):
     pattern, xy = hub_pattern(1300, 1400, 1399)
     n, _ = deal(pattern, xy, T)
     assert n < -512
+
+
+@pytest.mark.parametrize("n,nt", [(1, 1), (1, 8), (5, 8), (64, 8), (1000, 3)])
+def test_work_on_threads(lib, n, nt):
+    """Every piece once; an exception in one is told and ends no other thread's."""
+    assert lib.pieces(n, nt, -1) == n
+    assert -n < lib.pieces(n, nt, n // 2) <= 0
+
+
+def test_work_without_threads(lib):
+    """A process that cannot start another thread (stacks larger than its
+    address space may become) does the work on its own."""
+    import resource
+    import sys
+
+    def limits():
+        resource.setrlimit(resource.RLIMIT_STACK, (1 << 36, resource.RLIM_INFINITY))
+        resource.setrlimit(resource.RLIMIT_AS, (1 << 32, 1 << 32))
+    code = (f"import ctypes, threading\nlib = ctypes.CDLL({lib.path!r})\n"
+            "try:\n    threading.Thread(target=print).start()\n    print('started')\n"
+            "except RuntimeError:\n    print(lib.pieces(64, 8, -1))")
+    r = subprocess.run([sys.executable, "-c", code], preexec_fn=limits, capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.split() == ["64"], (r.returncode, r.stdout, r.stderr)
