@@ -97,7 +97,10 @@ inline void team_basin(const int *rowptr, const int *col, const float *xy, int k
                        TeamBasin &B) {
   const int K = sh.entries;
   std::vector<PlaneRow> v(nk);
-  for (int j = 0; j < nk; j++) v[j] = PlaneRow{{xy[2 * (size_t)(k0 + j)], xy[2 * (size_t)(k0 + j) + 1]}, k0 + j};
+  for (int j = 0; j < nk; j++) {         // NaN has no place in the order that bisect_rows needs
+    const float *p = xy + 2 * (size_t)(k0 + j);
+    v[j] = PlaneRow{{p[0] == p[0] ? p[0] : 0.f, p[1] == p[1] ? p[1] : 0.f}, k0 + j};
+  }
   B.cut.assign(T + 1, nk);
   bisect_rows(v.data(), nk, 0, 0, T, B.cut.data());
   std::vector<int> own(nk), place(nk), seen(nk, -1), gplace(nk), gl;

@@ -147,3 +147,19 @@ def test_work_without_threads(lib):
             "except RuntimeError:\n    print(lib.pieces(64, 8, -1))")
     r = subprocess.run([sys.executable, "-c", code], preexec_fn=limits, capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.split() == ["64"], (r.returncode, r.stdout, r.stderr)
+
+
+@pytest.mark.parametrize("T", [2, 7])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_coordinates_that_are_no_numbers(deal, bad, T):
+    """Nodes without coordinates (NaN; such as no element uses) are dealt
+    like nodes at the origin; infinite ones by their order."""
+    pattern, xy = hub_pattern(100, 1400, 1399)
+    rng = np.random.default_rng(5)
+    xy[rng.random(1400) < 0.3, 0] = bad
+    xy[rng.random(1400) < 0.3, 1] = bad
+    n, out = deal(pattern, xy, T, ghosts=1024)
+    check(pattern, n, out)
+    if np.isnan(bad):
+        m, want = deal(pattern, np.nan_to_num(xy), T, ghosts=1024)
+        assert m == n and all(np.array_equal(a, b) for a, b in zip(out, want))
