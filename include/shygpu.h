@@ -378,12 +378,15 @@ int shygpu_set_bound_scalar(shygpu_model *model, int32_t ibasin, int32_t what,
  * memory; 1, 2 one device-wide cooperative solve: the resident solver, or
  * the streaming one when a basin does not fit it), "zeta_stage" (streaming
  * solve with TMA-staged tiles), "inner_rtol" (residual reduction of each
- * FP32 Krylov sweep, default 1e-4), "inner_tol_frac" (an FP32 sweep also stops at this
- * fraction of the outer target, default 0.75), "max_outer" (FP64
- * refinement sweeps), "symmetric" (CG instead of BiCGStab; refused when
- * Coriolis makes the system non-symmetric), "column_threads" (1 one thread
- * per element column (with Coriolis for up to 16 layers), 0 one warp
- * segment),
+ * FP32 Krylov sweep, default 1e-4; the resident solver's CG goes to a tenth
+ * of it), "inner_tol_frac" (an FP32 sweep also stops at this fraction of the
+ * outer target, default 0.75), "max_outer" (FP64 refinement sweeps),
+ * "symmetric" (CG instead of BiCGStab; refused when Coriolis makes the
+ * system non-symmetric), "column_threads" (1 one thread per element column
+ * (with Coriolis for up to 16 layers), 0 one warp segment), "column_staged"
+ * and "node_prefetch" (forms of the thread-per-column kernels up to 16
+ * layers: columns staged in shared memory, an element's layers loaded at
+ * once),
  * "zeta_tile_rows" (rows per tile of the streaming solver, default 1024;
  * another value selects it),
  * "zeta_barrier_timeout_test" (failure detection: the device-wide solve's

@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(256) k_stab(Dev d, const int *kbas) {
 // nodes, one CTA each (blockIdx.y) of every basin (blockIdx.x: a grid has at
 // most 65535 CTAs in y); the CTA that finishes a basin last adds the chunks'
 // sums in order, so a basin's sums depend on it alone.  One CTA per basin took 162 us on 250k nodes (the
-// latency of 244 dependent loads a thread); the chunks take 33 us.
+// latency of 244 dependent loads a thread); the chunks take 31 us.
 // ===========================================================================
 constexpr int kReduceChunk = 4096;
 

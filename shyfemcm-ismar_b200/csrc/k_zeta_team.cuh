@@ -37,12 +37,11 @@
 // before they reached the share would bring it back.
 //
 // Measured (a solve, CUDA events; before: shared-memory clusters up to 40k
-// rows, the streaming solver above): 793 rows 51 iterations 268 -> 103 us,
-// 7k rows 121 iterations 615 -> 315 us, 20k rows 636 -> 360 us, 90k rows
-// 1156 -> 522 us, 250k rows 1139 -> 415 us, the 64-basin ensemble (2.1M rows)
-// 5.05 -> 2.71 ms; BiCGStab, 12k rows with Coriolis, 55 iterations 2.65 ->
-// 0.35 ms; the non-hydrostatic pressure (14k rows of up to 26 entries) 60 ->
-// 7 us an iteration.  What is left of an iteration (2 to 4 us) is a chain of
+// rows, the streaming solver above): 793 rows 52 iterations 268 -> 100 us,
+// 7k rows 122 iterations 615 -> 293 us, 20k rows 636 -> 355 us, 90k rows
+// 1156 -> 518 us, 250k rows 1139 -> 390 us, the 64-basin ensemble (2.1M rows)
+// 5.05 -> 2.65 ms; BiCGStab, 12k rows with Coriolis, 55 iterations 2.65 ->
+// 0.34 ms; the non-hydrostatic pressure (18k rows) 60 -> 7 us an iteration.  What is left of an iteration (2 to 4 us) is a chain of
 // latencies: the gathers 0.5 us, the sums in the CTA and the FP64 scalars
 // 0.6 us, one exchange through L2 0.5 us for a few members, 1 us for many.
 //

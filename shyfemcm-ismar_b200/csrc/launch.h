@@ -123,16 +123,17 @@ struct TeamMember {
   int row0, nrow, ghost0, nghost;
 };
 
-// the resident zeta solver.  Member m is worked by one CTA (cptr/clist, in
-// one order of the basins common to all CTAs).  Per row of the shares, in
-// their order: the global row (sign bit: some other member holds a ghost of
-// it), the place of the diagonal among the row's CSR slots with the count
-// of the others (dpos: dpos_pack), and the share's local column
-// (own rows, from zeta_team_rows() on the ghosts) of the first eight off-diagonal entries (lcol, as
-// byte offsets into a float array; the row itself on padding); rows with more keep the rest in a tail (tptr,
-// tcol, tslot, tval; null when no row has one).  word: four exchange buffers
-// of one word per row; part: two buffers of a
-// slot per member and the phantom, for its own sums and for the totals.
+// the resident solver.  Member m is worked by one CTA (cptr/clist, in one
+// order of the basins common to all CTAs).  Per row of the shares, in their
+// order: the global row (sign bit: some other member holds a ghost of it),
+// the place of the diagonal among the row's CSR slots with the count of the
+// others (dpos_pack), and the share's local columns (own rows, from
+// TeamShape::rows on the ghosts) of the first TeamShape::entries
+// off-diagonal entries (lcol, as byte offsets into a float array; the row
+// itself on padding); rows with more keep the rest in a tail (tptr, tcol,
+// tslot, tval; null when no row has one).  word: four exchange buffers of one
+// word per row; part: two buffers of a slot per member and the phantom, for
+// its own sums and for the totals.
 struct TeamPlan {
   // the system of the CSR instance: FP64 matrix and right-hand side, solution
   struct { const int *rowptr; const double *val, *rhs; float *x; } csr = {nullptr, nullptr, nullptr, nullptr};

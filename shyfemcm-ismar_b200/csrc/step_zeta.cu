@@ -63,8 +63,8 @@ cudaError_t launch_zeta_grid(const Dev &d, const ZetaArgs &za, const GridPlan &g
 constexpr int kTeamNT = 512;
 constexpr long long kTeamSpinLimit = 1LL << 22;   // polls of a word: seconds
 // the zeta system (rows of up to eight neighbours in the block), and the 3D
-// system (three layers of them and the two of the own column, less the row
-// itself, for up to eight neighbours)
+// system (a row has its node's neighbours at the same layer and the two
+// layers beside it, so most need 8 of the 26 places; longer ones have a tail)
 constexpr auto kZetaSym = k_zeta_team<kTeamNT, 4, 1, 8, true, false>;
 constexpr auto kZetaGen = k_zeta_team<kTeamNT, 4, 1, 8, false, false>;
 constexpr auto kCsrGen = k_zeta_team<kTeamNT, 1, 2, 26, false, true>;
@@ -102,12 +102,16 @@ TeamShape zeta_team_shape() {
   return TeamShape{kTeamNT * 4, kTeamNT, 8, std::min(team_capacity(kZetaSym), team_capacity(kZetaGen))};
 }
 TeamShape csr_team_shape() { return TeamShape{kTeamNT, 2 * kTeamNT, 26, team_capacity(kCsrGen)}; }
-// Rows a CTA gets: 1024 in small basins, where a team's latency matters (7k
-// rows: 0.31 ms a solve on 7 CTAs, 0.38 ms on 4), 2048 in larger ones, where
-// more members only make the exchange slower (250k rows: 0.42 ms on 123
-// CTAs, 0.66 ms on 245) and many basins take turns on the CTAs (the 64-basin
-// ensemble: 2.8 ms with 2048 rows everywhere, 3.6 ms with 1024 up to 40k
-// rows).  It depends on the basin alone, so that its bits do.
+// Rows a CTA gets.  Basins alone are faster in shares of 1024 rows than of
+// 2048 (us a solve by CG: 3k rows 157 against 165, 7k 161/191, 12k 162/201,
+// 20k 170/204, 36k 190/213, 60k 192/215, 90k 208/243; at 150k, 147 members,
+// 271/258), many basins in one model in larger ones, whose teams take fewer
+// turns on the CTAs (24 basins of 9000 rows 348 against 224, 24 of 20000
+// 712/453, 16 members of the ensemble 1405/648, all 64 5100/2500).  A basin's
+// bits may depend on the basin alone, so the rule cannot ask how many there
+// are: small basins, which are run alone, get 1024 rows and pay 55% more
+// where two dozen share a model; larger ones 2048, at 10 to 20% of their
+// time alone.  The line between them lies at no knee of either curve.
 int zeta_team_share(int nk) { return nk <= 12288 ? kTeamNT * 2 : kTeamNT * 4; }
 long long zeta_team_spin_limit() { return kTeamSpinLimit; }
 
